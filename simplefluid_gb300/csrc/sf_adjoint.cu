@@ -58,6 +58,14 @@ __device__ __forceinline__ float dot3f(float ax, float ay, float az, float bx, f
     return fmaf(az, bz, fmaf(ay, by, ax * bx));
 }
 
+// A step's gather record as (x, y, z, p), (vx, vy, vz, 1/rho).
+__device__ __forceinline__ void ld_state(const float4* __restrict__ p, float4& x, float4& v) {
+    float4 a, b;
+    ld8(p, a, b);
+    x = make_float4(a.x, a.z, b.x, b.z);
+    v = make_float4(a.y, a.w, b.y, b.w);
+}
+
 // P1: per sorted particle.  Outputs the 32-byte record abrec = apb (cp tb,
 // inv_bar), avb (cv tb, cv_bar), and xdir/vdir = the integration's direct
 // adjoints.
@@ -127,7 +135,7 @@ __device__ __forceinline__ void eos_derivs(const SimConst& c, float rho, float& 
 // adjoint of the particle.  Outputs xrb = (x, y, z, rho_bar), P4's gather
 // record, xf = (force x_bar, k_bar) and vf.
 // A neighbour is two 32-byte records, each one 256-bit load: the step's
-// (x, y, z, p | vx, vy, vz, 1/rho) and P1's (apb | avb).
+// gather record and P1's (apb | avb).
 template <int kReach>
 __global__ void __launch_bounds__(kAdjBlock)
     k_adj_forces(const float4* __restrict__ pos, const float4* __restrict__ pv, const float2* __restrict__ pr,
@@ -137,7 +145,7 @@ __global__ void __launch_bounds__(kAdjBlock)
     const uint32_t k = blockIdx.x * kAdjBlock + threadIdx.x;
     if (k >= n) return;
     float4 xk, vk, apbk, avbk;
-    ld8(pv + 2 * (size_t)k, xk, vk);
+    ld_state(pv + 2 * (size_t)k, xk, vk);
     ld8(ab + 2 * (size_t)k, apbk, avbk);
     const float2 prk = pr[k];
     const float pk = prk.x, invk = prk.y;
@@ -205,7 +213,7 @@ __global__ void __launch_bounds__(kAdjBlock)
         uint32_t jc = checked_index(__ldg(lst), n), jn = __ldg(lst + kNbTile);
         float4 nx, nv, na, nb;
         if (m) {
-            ld8(pv + 2 * (size_t)jc, nx, nv);
+            ld_state(pv + 2 * (size_t)jc, nx, nv);
             ld8(ab + 2 * (size_t)jc, na, nb);
         }
         for (uint32_t s = 0; s < m; ++s) {
@@ -214,7 +222,7 @@ __global__ void __launch_bounds__(kAdjBlock)
             if (s + 1 < m) {
                 jc = checked_index(jn, n);
                 jn = __ldg(lst + (size_t)min(s + 2, (uint32_t)kNbCap - 1) * kNbTile);
-                ld8(pv + 2 * (size_t)jc, nx, nv);
+                ld_state(pv + 2 * (size_t)jc, nx, nv);
                 ld8(ab + 2 * (size_t)jc, na, nb);
             }
             if (j != k) pair(xj, vj, apbj, avbj);
@@ -225,7 +233,7 @@ __global__ void __launch_bounds__(kAdjBlock)
             const float dx = xk.x - xp.x, dy = xk.y - xp.y, dz = xk.z - xp.z;
             if (!(fmaf(dz, dz, fmaf(dy, dy, dx * dx)) < c.h2)) return;
             float4 xj, vj, apbj, avbj;
-            ld8(pv + 2 * (size_t)j, xj, vj);
+            ld_state(pv + 2 * (size_t)j, xj, vj);
             ld8(ab + 2 * (size_t)j, apbj, avbj);
             pair(xj, vj, apbj, avbj);
         });

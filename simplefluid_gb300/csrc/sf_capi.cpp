@@ -241,7 +241,7 @@ sf_status alloc_particles(sf_ctx* ctx, uint32_t n) {
     if (e == cudaSuccess) e = dev_malloc(&d.key_slot, c * sizeof(uint2));
     if (e == cudaSuccess) e = dev_malloc(&d.tmp, c * sizeof(uint32_t));
     if (e == cudaSuccess) e = dev_malloc(&d.io, c * 6 * sizeof(float));
-    if (e == cudaSuccess) e = dev_malloc(&d.nbr, tiles * sf::kNbCap * sf::kNbTile * sizeof(uint32_t));
+    if (e == cudaSuccess) e = dev_malloc(&d.nbr, sf::nbr_entries(c) * sizeof(uint32_t));
     if (e == cudaSuccess) e = dev_malloc(&d.nbr_count, c * sizeof(uint32_t));
     if (e == cudaSuccess) e = dev_malloc(&d.nbr_wide, tiles * (sf::kNbTile / sf::kNbWarpTile));
     if (e == cudaSuccess) e = dev_malloc(&d.pv, c * 2 * sizeof(float4));

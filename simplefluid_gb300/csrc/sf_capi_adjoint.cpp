@@ -37,7 +37,6 @@ sf_status ensure_work(sf_ctx* ctx) {
 sf_status ensure_records(sf_ctx* ctx, uint32_t ckpt) {
     sf::Trajectory* t = ctx->traj;
     const size_t n = ctx->d.cap;
-    const size_t tiles = (n + sf::kNbTile - 1) / sf::kNbTile;
     if (t->rec.size() == ckpt && t->ncells_pad == ctx->d.ncells_pad && t->stage) return SF_OK;
     drop_segment_graphs(t);
     for (auto& r : t->rec) free_rec(r);
@@ -54,7 +53,7 @@ sf_status ensure_records(sf_ctx* ctx, uint32_t ckpt) {
         SF_ALLOC_TRAJ(r.vel, n * sizeof(float4));
         SF_ALLOC_TRAJ(r.pr, n * sizeof(float2));
         SF_ALLOC_TRAJ(r.rho, n * sizeof(float));
-        SF_ALLOC_TRAJ(r.nbr, tiles * sf::kNbCap * sf::kNbTile * sizeof(uint32_t));
+        SF_ALLOC_TRAJ(r.nbr, sf::nbr_entries(n) * sizeof(uint32_t));
         SF_ALLOC_TRAJ(r.cnt, n * sizeof(uint32_t));
         SF_ALLOC_TRAJ(r.cs, (size_t)ctx->d.ncells_pad * sizeof(uint32_t));
         SF_ALLOC_TRAJ(r.sums, 2 * n * sizeof(float4));

@@ -4,7 +4,7 @@
 // candidates; non-neighbours add an exact zero (fma(0, 0, s) == s), so the sum
 // is branch-free and bit-identical to summing neighbours only.  The pass also
 // evaluates the equation of state, writes each particle's 32-byte record for
-// the force pass's gathers ((x, y, z, p), (vx, vy, vz, 1/rho)), and records
+// the force pass's gathers ((x, vx, y, vy), (z, vz, p, 1/rho)), and records
 // each particle's neighbours (itself included, in its canonical place) for the
 // force pass:
 //   kEmitNone    no list (the force pass rescans the candidate cells);

@@ -450,8 +450,7 @@ __device__ __forceinline__ size_t nbr_w16_index(uint32_t i, uint32_t k) {
     return ((size_t)(i / kNbWarpTile) * (2 * kNbCap) + k) * kNbWarpTile + (i % kNbWarpTile);
 }
 
-// Pair terms of particle i with neighbour j (|xi - xj| < h; j == i adds exact
-// zeros), in the oracle's operation order.
+// The force sums of one particle: AP (pressure) and AV (viscosity).
 struct PairAcc {
     float apx = 0.f, apy = 0.f, apz = 0.f, avx = 0.f, avy = 0.f, avz = 0.f;
 };
@@ -465,6 +464,147 @@ __device__ __forceinline__ const T* opaque_ptr(const T* p) {
     return r;
 }
 
+// Two floats in one register pair, and the sm_100+ instructions that work on
+// both halves (each half an IEEE operation, rounded to nearest).
+struct F2 {
+    unsigned long long v;
+};
+__device__ __forceinline__ F2 f2(float lo, float hi) {
+    F2 r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r.v) : "f"(lo), "f"(hi));
+    return r;
+}
+__device__ __forceinline__ float2 unpack(F2 a) {
+    float2 r;
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(a.v));
+    return r;
+}
+__device__ __forceinline__ F2 add2(F2 a, F2 b) {
+    F2 r;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r.v) : "l"(a.v), "l"(b.v));
+    return r;
+}
+__device__ __forceinline__ F2 mul2(F2 a, F2 b) {
+    F2 r;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r.v) : "l"(a.v), "l"(b.v));
+    return r;
+}
+__device__ __forceinline__ F2 fma2(F2 a, F2 b, F2 c) {
+    F2 r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r.v) : "l"(a.v), "l"(b.v), "l"(c.v));
+    return r;
+}
+__device__ __forceinline__ float rsqrt_approx(float x) {
+    float y;
+    asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+    return y;
+}
+
+// The range of the list gather's own root and quotient (pair_terms2).  With
+// the kernel radius inside [kFastHMin, kFastHMax] and the squared distance
+// zero or at least kFastR2Min, every step of them is a normal number and the
+// results are the correctly rounded ones.
+constexpr float kFastR2Min = 8.0779357e-28f;  // 2^-90
+constexpr float kFastHMin = 3.8146973e-06f;   // 2^-18: h - 2^-45 rounds to h
+constexpr float kFastHMax = 1.0995116e+12f;   // 2^40
+
+// Pair sums of one particle over its list, two neighbours at a time.  The
+// gather record's order (x, vx, y, vy, z, vz, p, 1/rho) puts a position
+// component beside the velocity component that the same packed instruction
+// subtracts and accumulates: (x, vx)_i - (x, vx)_j and (AP, AV) += (-sp, w) *
+// difference.
+struct PairSums {
+    F2 x, y, z;      // (apx, avx), (apy, avy), (apz, avz)
+    F2 nx, ny, nz;   // -(x, vx), -(y, vy), -(z, vz) of the particle itself
+    float p;         // its pressure
+    uint32_t small;  // min over the pairs of bits(r^2) - 1: below bits(kFastR2Min) - 1 some r^2 was tiny but not 0
+};
+__device__ __forceinline__ void start_sums(PairSums& a, const float4& xi, const float4& vi, float pi) {
+    a.x = a.y = a.z = f2(0.f, 0.f);
+    a.nx = f2(-xi.x, -vi.x);
+    a.ny = f2(-xi.y, -vi.y);
+    a.nz = f2(-xi.z, -vi.z);
+    a.p = pi;
+    a.small = 0xffffffffu;
+}
+// A gather record as its four pairs.
+struct PairRec {
+    F2 x, y, z, pw;  // (x, vx), (y, vy), (z, vz), (p, 1/rho)
+};
+
+// A gather record in one access.
+template <bool kNc>
+__device__ __forceinline__ void ld_rec(const float4* __restrict__ p, PairRec& r) {
+    if constexpr (kNc)
+        asm volatile("ld.global.nc.v4.b64 {%0, %1, %2, %3}, [%4];"
+                     : "=l"(r.x.v), "=l"(r.y.v), "=l"(r.z.v), "=l"(r.pw.v)
+                     : "l"(p));
+    else
+        asm volatile("ld.global.v4.b64 {%0, %1, %2, %3}, [%4];"
+                     : "=l"(r.x.v), "=l"(r.y.v), "=l"(r.z.v), "=l"(r.pw.v)
+                     : "l"(p));
+}
+
+// The distance and its quotient of two pairs, from their r^2.  They are not
+// the compiler's root and division: those branch on their operand's range,
+// which keeps two neighbours' chains from interleaving, and start from two
+// separate approximations.  Here both come from one approximation of
+// 1/sqrt(r^2): a Newton step in residual form for the root, one for its
+// reciprocal, then Markstein's quotient correction (P. Markstein, "Computation
+// of elementary functions on the IBM RISC System/6000 processor", 1990), all
+// on both pairs at once.  Over the stated range the results are the IEEE ones:
+// checked for every float r^2 (root), and for every quotient close enough to a
+// rounding boundary to be in doubt (118,635,758 numerators over all roots; the
+// error before the last rounding is under 1.5 * 2^-24 of a unit, so a quotient
+// further than that from a boundary cannot round wrong).
+// A coincident neighbour (r^2 = 0, the particle itself included) takes
+// r = 2^-45, so that h - r == h.
+struct RootQuotient {
+    F2 hr;      // h - r
+    float2 nq;  // -(h - r) / r
+};
+__device__ __forceinline__ RootQuotient root_quotient(F2 hh, float ra, float rb) {
+    const float ca = fmaxf(ra, kFastR2Min), cb = fmaxf(rb, kFastR2Min);
+    const F2 n2 = f2(-ca, -cb), y0 = f2(rsqrt_approx(ca), rsqrt_approx(cb));
+    const F2 ns = mul2(n2, y0);                             // -r^2 y0
+    const F2 d = fma2(ns, ns, n2);                          // residual (r^2 y0)^2 - r^2
+    const F2 nr = fma2(d, mul2(y0, f2(0.5f, 0.5f)), ns);    // -r
+    // 1 / r; the 2^-45 settles the one reciprocal that this step would round
+    // down (r one place below a power of two)
+    const F2 e = add2(fma2(nr, y0, f2(1.f, 1.f)), f2(2.8421709e-14f, 2.8421709e-14f));
+    const F2 y = fma2(e, y0, y0);
+    RootQuotient o;
+    o.hr = add2(hh, nr);
+    const F2 q0 = mul2(o.hr, y);
+    const float2 q = unpack(fma2(fma2(nr, q0, o.hr), y, q0));
+    o.nq = make_float2(-q.x, -q.y);
+    return o;
+}
+__device__ __forceinline__ float square3(F2 x, F2 y, F2 z) {  // of the low halves
+    const float dx = unpack(x).x, dy = unpack(y).x, dz = unpack(z).x;
+    return fmaf(dz, dz, fmaf(dy, dy, dx * dx));
+}
+// Terms of two neighbours, the first one's added before the second one's, in
+// the oracle's operation order.  A coincident neighbour's differences are
+// zeros, and its pressure weight is set to zero as in pair_terms.
+__device__ __forceinline__ void pair_terms2(F2 hh, const PairRec& a, const PairRec& b, PairSums& s) {
+    const F2 ax = add2(a.x, s.nx), ay = add2(a.y, s.ny), az = add2(a.z, s.nz);  // (xj - xi, vj - vi)
+    const F2 bx = add2(b.x, s.nx), by = add2(b.y, s.ny), bz = add2(b.z, s.nz);
+    const float ra = square3(ax, ay, az), rb = square3(bx, by, bz);
+    s.small = min(s.small, min(__float_as_uint(ra) - 1u, __float_as_uint(rb) - 1u));
+    const RootQuotient t = root_quotient(hh, ra, rb);
+    const float2 hr = unpack(t.hr), pa = unpack(a.pw), pb = unpack(b.pw);
+    const float wa = hr.x * pa.y, wb = hr.y * pb.y;
+    const float sa = ((s.p + pa.x) * wa) * t.nq.x, sb = ((s.p + pb.x) * wb) * t.nq.y;
+    const F2 ka = f2(ra > 0.f ? sa : 0.f, wa), kb = f2(rb > 0.f ? sb : 0.f, wb);
+    s.x = fma2(kb, bx, fma2(ka, ax, s.x));
+    s.y = fma2(kb, by, fma2(ka, ay, s.y));
+    s.z = fma2(kb, bz, fma2(ka, az, s.z));
+}
+
+// Terms of particle i with neighbour j (|xi - xj| < h; j == i adds exact
+// zeros) with the compiler's root and division, at any kernel radius and
+// distance.
 __device__ __forceinline__ void pair_terms(float h, const float4& xi, const float4& vi, float pi,
                                            const float4& xj, const float2& prj, const float4& vj, PairAcc& a) {
     const float dx = xi.x - xj.x, dy = xi.y - xj.y, dz = xi.z - xj.z;

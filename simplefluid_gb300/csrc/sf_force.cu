@@ -7,7 +7,7 @@
 // variant, symplectic Euler, the box clamp with restitution and the next
 // step's cell key and arrival slot (the counting sort's histogram).
 // A neighbour on the list is one 32-byte record written by the density pass,
-// (x, y, z, p) and (vx, vy, vz, 1/rho), fetched with one 256-bit load.
+// (x, vx, y, vy) and (z, vz, p, 1/rho), fetched with one 256-bit load.
 // kPrefetch neighbours are gathered before their terms are added, and the
 // next kPrefetch list entries are loaded while they are, so the dependent
 // index -> data loads of consecutive batches overlap; the terms are still
@@ -19,8 +19,34 @@
 namespace sf {
 namespace {
 
+// Raises the frame's maxima of |v'|^2 and |a|^2 to those of the block
+// (non-negative floats order like their bits), with one atomic each per block.
+template <int kBlockSize>
+__device__ __forceinline__ void raise_maxima(FrameState* __restrict__ frame, uint32_t v2, uint32_t a2) {
+    __shared__ uint32_t s_max[2][kBlockSize / 32];
+    v2 = __reduce_max_sync(0xffffffffu, v2);
+    a2 = __reduce_max_sync(0xffffffffu, a2);
+    if ((threadIdx.x & 31) == 0) {
+        s_max[0][threadIdx.x / 32] = v2;
+        s_max[1][threadIdx.x / 32] = a2;
+    }
+    __syncthreads();
+    if (threadIdx.x < 32) {
+        const bool have = threadIdx.x < kBlockSize / 32;
+        const uint32_t mv = __reduce_max_sync(0xffffffffu, have ? s_max[0][threadIdx.x] : 0u);
+        const uint32_t ma = __reduce_max_sync(0xffffffffu, have ? s_max[1][threadIdx.x] : 0u);
+        if (threadIdx.x == 0) {
+            atomicMax(&frame->v2max_bits, mv);
+            atomicMax(&frame->a2max_bits, ma);
+        }
+    }
+}
+
+// Registers are capped at 56 (nine blocks of 128 threads per SM; 58 would fit
+// only eight: 100 us instead of 95 at 1,048,576 particles) or, with four
+// gathers in flight, at 72 (seven blocks).
 template <int kList, int kPrefetch, int kBlockSize, bool kIntegrate, int kReach, bool kBatched>
-__global__ void __launch_bounds__(kBlockSize)
+__global__ void __launch_bounds__(kBlockSize, (kPrefetch == 2 ? 1152 : 896) / kBlockSize)
     k_force(const float4* __restrict__ pos, const float4* __restrict__ vel, const float2* __restrict__ pr,
             const uint32_t* __restrict__ cs, const uint32_t* __restrict__ nbr, const uint32_t* __restrict__ nbr_count,
             const uint8_t* __restrict__ nbr_wide, const float4* __restrict__ pv, uint32_t n, SimConst c0, const SimConst* __restrict__ table, const uint32_t* __restrict__ scene_off,
@@ -36,27 +62,7 @@ __global__ void __launch_bounds__(kBlockSize)
                                                                   table,
                                                                      scene_off, nscenes, pos_out, vel_out, counts,
                                                                      tile_sums, key_slot, acc_out, sums, frame, v2, a2);
-    if (!kBatched && kIntegrate && frame && c0.adaptive) {
-        // maxima of |v'|^2 and |a|^2 over the block (non-negative floats order
-        // like their bits), then one atomic each per block
-        __shared__ uint32_t s_max[2][kBlockSize / 32];
-        v2 = __reduce_max_sync(0xffffffffu, v2);
-        a2 = __reduce_max_sync(0xffffffffu, a2);
-        if ((threadIdx.x & 31) == 0) {
-            s_max[0][threadIdx.x / 32] = v2;
-            s_max[1][threadIdx.x / 32] = a2;
-        }
-        __syncthreads();
-        if (threadIdx.x < 32) {
-            const bool have = threadIdx.x < kBlockSize / 32;
-            const uint32_t mv = __reduce_max_sync(0xffffffffu, have ? s_max[0][threadIdx.x] : 0u);
-            const uint32_t ma = __reduce_max_sync(0xffffffffu, have ? s_max[1][threadIdx.x] : 0u);
-            if (threadIdx.x == 0) {
-                atomicMax(&frame->v2max_bits, mv);
-                atomicMax(&frame->a2max_bits, ma);
-            }
-        }
-    }
+    if (!kBatched && kIntegrate && frame && c0.adaptive) raise_maxima<kBlockSize>(frame, v2, a2);
 }
 
 template <int kList, int kPrefetch, int kBlockSize, bool kIntegrate>

@@ -59,6 +59,22 @@ int scene_points(const sf_params& p, int scene, uint64_t seed, std::vector<float
 int batch_cubes(uint64_t seed, uint32_t nscenes, const sf_params& base, std::vector<sf_params>& params,
                 std::vector<uint32_t>& counts, std::vector<float>& pos, const char** why);
 
+// Neighbour lists: up to kNbCap neighbours per particle, in tiles of kNbTile
+// particles (see nbr_index in sf_device.cuh).  A buffer for n particles holds
+// nbr_entries(n) entries.
+constexpr int kNbTile = 128;
+constexpr int kNbCap = 64;
+// Entries past the last tile: the force pass loads two slots ahead of a list's
+// end (and uses none of them).
+constexpr int kNbSlack = 2 * kNbTile;
+constexpr int kNbWarpTile = 32;  // tiles of SF_LIST_TILE16 lists: one warp's particles
+constexpr size_t nbr_entries(size_t n) { return (n + kNbTile - 1) / kNbTile * kNbCap * kNbTile + kNbSlack; }
+// list emission modes of the density pass
+constexpr int kEmitNone = 0, kEmitStaged = 1, kEmitTile = 2, kEmitTile16 = 3;
+// SF_LIST_TILE16: entries hold the neighbour index's low 16 bits, exact when
+// |j - i| <= kNear16 (j = i + (int16_t)(entry - i)).
+constexpr uint32_t kNear16 = 32767;
+
 // Kernel choices of a context (all give bit-identical results).
 struct Tuning {
     int list_mode = SF_LIST_TILE;  // SF_LIST_*: how the density pass records neighbours
@@ -87,7 +103,7 @@ struct DeviceState {
     uint32_t* nbr = nullptr;       // neighbour lists, tile-major (kNbCap * kNbTile per tile)
     uint32_t* nbr_count = nullptr; // neighbours of each particle (may exceed kNbCap)
     uint8_t* nbr_wide = nullptr;   // SF_LIST_TILE16: per warp tile (kNbWarpTile particles), 1 where it holds 32-bit entries
-    float4* pv = nullptr;          // 2 per particle (32 bytes): (x, y, z, p), (vx, vy, vz, 1/rho)
+    float4* pv = nullptr;          // 2 per particle (32 bytes): (x, vx, y, vy), (z, vz, p, 1/rho)
     float4* sums = nullptr;        // optional: per particle (AP, 0), (AV, 0) of the force pass (adjoint recording)
     FrameState* frame = nullptr;   // adaptive sub-steps read dt here and raise the maxima
     // grid
@@ -107,17 +123,6 @@ struct DeviceState {
     const uint32_t* scene_order = nullptr;
     uint32_t* scene_queue = nullptr;
 };
-
-// Neighbour lists: up to kNbCap neighbours per particle, in tiles of kNbTile
-// particles (see nbr_index in sf_device.cuh).
-constexpr int kNbTile = 128;
-constexpr int kNbCap = 64;
-constexpr int kNbWarpTile = 32;  // tiles of SF_LIST_TILE16 lists: one warp's particles
-// list emission modes of the density pass
-constexpr int kEmitNone = 0, kEmitStaged = 1, kEmitTile = 2, kEmitTile16 = 3;
-// SF_LIST_TILE16: entries hold the neighbour index's low 16 bits, exact when
-// |j - i| <= kNear16 (j = i + (int16_t)(entry - i)).
-constexpr uint32_t kNear16 = 32767;
 
 constexpr int kScanThreads = 1024;
 constexpr int kScanItems = 4;
@@ -212,7 +217,7 @@ struct AdjointStep {
     const uint32_t* cnt = nullptr;
     const uint32_t* cs = nullptr;
     const float4* sums = nullptr;
-    const float4* pv = nullptr;  // the step's 32-byte gather records (x, y, z, p), (vx, vy, vz, 1/rho)
+    const float4* pv = nullptr;  // the step's 32-byte gather records (x, vx, y, vy), (z, vz, p, 1/rho)
 };
 // Adjoint working buffers (N particles).  Xb/Vb are indexed by particle id.
 struct AdjointWork {
