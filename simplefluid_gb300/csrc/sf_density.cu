@@ -25,8 +25,9 @@
 // candidates instead of reading the list.  Recording the particle itself saves
 // a comparison per candidate; its pair terms in the force pass are exact
 // zeros (fma(w, v_i - v_i, a) == a, and the pressure term needs r > 0).
-// The per-particle pass itself (density_one) is in sf_passes.cuh.
-#include "sf_passes.cuh"
+// The per-particle pass itself (density_one) is in sf_passes.cuh; small scenes
+// take the team form of sf_team.cuh.
+#include "sf_team.cuh"
 
 namespace sf {
 namespace {
@@ -67,6 +68,20 @@ __global__ void __launch_bounds__(kBlockSize)
     }
 }
 
+template <int kReach>
+__global__ void __launch_bounds__((2 * kReach + 1) * 32)
+    k_density_team(const float4* __restrict__ pos, const uint32_t* __restrict__ cs, uint32_t n, SimConst c,
+                   float* __restrict__ rho_out, float2* __restrict__ pr_out, uint32_t* __restrict__ nbr,
+                   uint32_t* __restrict__ nbr_count, const float4* __restrict__ vel, float4* __restrict__ pv,
+                   FrameState* __restrict__ frame) {
+    __shared__ DensityTeamShared<kReach> sh;
+    grid_dependency_wait();
+    allow_dependents();
+    if (frame && blockIdx.x == 0 && threadIdx.x == 0) choose_dt(frame, c);
+    const uint32_t i = blockIdx.x * kTeamParticles + (threadIdx.x & 31u);
+    density_team<kReach>(min(i, n - 1), i < n, c, pos, cs, n, rho_out, pr_out, nbr, nbr_count, vel, pv, sh);
+}
+
 template <int kMode, int kBlockSize>
 void density_as(const DeviceState& d, const SimConst& c, cudaStream_t s) {
     // the gather records are written here and gathered by the force pass
@@ -94,8 +109,23 @@ void density_as(const DeviceState& d, const SimConst& c, cudaStream_t s) {
 
 SF_INDEX_CHECK_ACCESSOR(index_check_failures_density)
 
+bool standard_passes(const DeviceState& d) {
+    const Tuning standard;
+    return !d.table && d.nbr && d.tune.list_mode == standard.list_mode &&
+           d.tune.density_block == standard.density_block && d.tune.force_block == standard.force_block &&
+           !d.tune.l2_window;
+}
+
 void launch_density(const DeviceState& d, const SimConst& c, cudaStream_t s) {
     if (!d.n) return;
+    if (d.n < kDensityTeamScene && standard_passes(d)) {
+        with_reach(c.reach, [&](auto R) {
+            constexpr int K = decltype(R)::value;
+            launch_chained(k_density_team<K>, grid_for(d.n, kTeamParticles), (2 * K + 1) * 32, s, d.pos, d.cell_start,
+                           d.n, c, d.rho, d.pr, d.nbr, d.nbr_count, d.vel, d.pv, d.frame);
+        });
+        return;
+    }
     const bool big = d.tune.density_block == 256;
     if (!d.nbr || d.tune.list_mode == SF_LIST_NONE) {
         big ? density_as<kEmitNone, 256>(d, c, s) : density_as<kEmitNone, 128>(d, c, s);

@@ -13,8 +13,9 @@
 // index -> data loads of consecutive batches overlap; the terms are still
 // added in list order, which keeps the sum bit-identical.  Lists of 16-bit
 // entries (SF_LIST_TILE16) are decoded to indices where they are used.  The
-// per-particle pass itself (force_one) is in sf_passes.cuh.
-#include "sf_passes.cuh"
+// per-particle pass itself (force_one) is in sf_passes.cuh; small scenes take
+// the team form of sf_team.cuh.
+#include "sf_team.cuh"
 
 namespace sf {
 namespace {
@@ -65,6 +66,56 @@ __global__ void __launch_bounds__(kBlockSize, (kPrefetch == 2 ? 1152 : 896) / kB
     if (!kBatched && kIntegrate && frame && c0.adaptive) raise_maxima<kBlockSize>(frame, v2, a2);
 }
 
+template <bool kIntegrate, int kReach, int kTeam, int kTurn>
+__global__ void __launch_bounds__(kTeam * 32)
+    k_force_team(const float4* __restrict__ pos, const float4* __restrict__ vel, const float2* __restrict__ pr,
+                 const uint32_t* __restrict__ cs, const uint32_t* __restrict__ nbr,
+                 const uint32_t* __restrict__ nbr_count, const float4* __restrict__ pv, uint32_t n, SimConst c,
+                 float4* __restrict__ pos_out, float4* __restrict__ vel_out, uint32_t* __restrict__ counts,
+                 uint32_t* __restrict__ tile_sums, uint2* __restrict__ key_slot, float4* __restrict__ acc_out,
+                 float4* __restrict__ sums, FrameState* __restrict__ frame) {
+    __shared__ ForceTeamShared sh;
+    grid_dependency_wait();
+    allow_dependents();
+    const uint32_t first = blockIdx.x * kTeamParticles + (threadIdx.x & 31u), i = min(first, n - 1);
+    float4 xi, vi;
+    float2 pri;
+    PairAcc a;
+    bool last;
+    const bool summed = force_team<kTeam, kTurn>(i, nbr_count, nbr, pv, n, c.h, sh, a, last, [&](bool finishes) {
+        if (finishes) {  // the warp that integrates the particles
+            xi = ldg4(pos + i);
+            vi = ldg4(vel + i);
+            pri = __ldg(pr + i);
+        }
+    });
+    uint32_t v2 = 0u, a2 = 0u;
+    if (last && first < n) {
+        if (!summed) {
+            a = PairAcc{};
+            force_rescan<kReach, true>(i, c, pos, vel, pr, cs, n, xi, vi, pri.x, a);
+        }
+        if (sums) {
+            sums[2 * (size_t)i] = make_float4(a.apx, a.apy, a.apz, 0.f);
+            sums[2 * (size_t)i + 1] = make_float4(a.avx, a.avy, a.avz, 0.f);
+        }
+        force_finish<kIntegrate>(i, c, xi, vi, pri.y, a, pos_out, vel_out, counts, tile_sums, key_slot, acc_out, frame,
+                                 v2, a2);
+    }
+    if (kIntegrate && frame && c.adaptive) raise_maxima<kTeam * 32>(frame, v2, a2);
+}
+
+template <bool kIntegrate, int kTeam, int kTurn>
+void force_team_as(DeviceState& d, const SimConst& c, cudaStream_t s) {
+    with_reach(c.reach, [&](auto R) {
+        launch_chained(k_force_team<kIntegrate, decltype(R)::value, kTeam, kTurn>, grid_for(d.n, kTeamParticles),
+                       kTeam * 32, s, d.pos, d.vel, d.pr, d.cell_start, d.nbr, d.nbr_count, d.pv, d.n, c,
+                       kIntegrate ? d.pos2 : nullptr, kIntegrate ? d.vel2 : nullptr, kIntegrate ? d.counts : nullptr,
+                       kIntegrate ? d.tile_sums : nullptr, kIntegrate ? d.key_slot : nullptr,
+                       kIntegrate ? nullptr : d.accel, d.sums, kIntegrate ? d.frame : nullptr);
+    });
+}
+
 template <int kList, int kPrefetch, int kBlockSize, bool kIntegrate>
 void force_as(DeviceState& d, const SimConst& c, cudaStream_t s) {
     cudaAccessPolicyWindow w{};
@@ -98,6 +149,10 @@ void force_as(DeviceState& d, const SimConst& c, cudaStream_t s) {
 template <bool kIntegrate>
 void launch_force(DeviceState& d, const SimConst& c, cudaStream_t s) {
     if (!d.n) return;
+    if (d.n < kForceTeamScene && standard_passes(d)) {
+        force_team_as<kIntegrate, kForceTeam, kForceTurn>(d, c, s);
+        return;
+    }
     const bool big = d.tune.force_block == 256;
     if (!d.nbr || d.tune.list_mode == SF_LIST_NONE) {
         big ? force_as<0, 2, 256, kIntegrate>(d, c, s) : force_as<0, 2, 128, kIntegrate>(d, c, s);

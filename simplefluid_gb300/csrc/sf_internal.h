@@ -162,6 +162,19 @@ void launch_scatter(const uint2* key_slot, const uint32_t* cell_start, uint32_t 
 void launch_rank_gather(const uint2* key_slot, const uint32_t* cell_start, const uint32_t* tmp, const float4* pos_in,
                         const float4* vel_in, uint32_t n, float4* pos_out, float4* vel_out, uint32_t* tile_sums,
                         uint32_t ntiles, cudaStream_t s);
+// Scenes of fewer particles take the team forms (sf_team.cuh) of the two
+// passes.  Stage times in us, one thread per particle against the team
+// (jittered lattice; disordered): density 16.4 / 10.3 at 16,000 particles,
+// 23.8 / 20.0; 25.1 / 23.9 at 56,000, 24.5 / 24.6 at 65,536 (disordered);
+// force 12.3 / 9.5 at 16,000, 12.9 / 12.3; 14.7 / 14.3 at 32,000, 13.1 / 16.1
+// at 48,000.
+constexpr uint32_t kDensityTeamScene = 57344, kForceTeamScene = 32768;
+// Warps per 32 particles in the force pass, and neighbours they take in turn
+// (2 x 4; stage times at 16,000 and 32,000 particles 9.5 and 12.3 us, 4 x 4
+// 9.6 and 13.7, 3 x 2 9.6 and 13.9, 8 x 2 12.4 and 15.6).
+constexpr int kForceTeam = 2, kForceTurn = 4;
+// Whether the step uses the default kernel choices on a single scene.
+bool standard_passes(const DeviceState& d);
 void launch_density(const DeviceState& d, const SimConst& c, cudaStream_t s);
 // forces + symplectic Euler + box + next-step cell hash into pos2/vel2
 void launch_force_integrate(DeviceState& d, const SimConst& c, cudaStream_t s);
