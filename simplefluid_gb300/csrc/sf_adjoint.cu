@@ -24,7 +24,7 @@
 namespace sf {
 namespace {
 
-constexpr int kAdjBlock = 128;
+constexpr int kAdjBlock = 128, kAdjForceBlock = 64;
 
 // Calls f(j, pos[j]) for the neighbours j != i (|xi - xj| < h) of sorted
 // particle i, in canonical order: from the recorded list, or by walking the
@@ -58,17 +58,9 @@ __device__ __forceinline__ float dot3f(float ax, float ay, float az, float bx, f
     return fmaf(az, bz, fmaf(ay, by, ax * bx));
 }
 
-// A step's gather record as (x, y, z, p), (vx, vy, vz, 1/rho).
-__device__ __forceinline__ void ld_state(const float4* __restrict__ p, float4& x, float4& v) {
-    float4 a, b;
-    ld8(p, a, b);
-    x = make_float4(a.x, a.z, b.x, b.z);
-    v = make_float4(a.y, a.w, b.y, b.w);
-}
-
-// P1: per sorted particle.  Outputs the 32-byte record abrec = apb (cp tb,
-// inv_bar), avb (cv tb, cv_bar), and xdir/vdir = the integration's direct
-// adjoints.
+// P1: per sorted particle.  Outputs the 32-byte record abrec = apb = cp tb
+// beside avb = cv tb in each axis, then (inv_bar, cv_bar); and xdir/vdir = the
+// integration's direct adjoints.
 __global__ void __launch_bounds__(kAdjBlock)
     k_adj_integrate(const float4* __restrict__ pos, const float4* __restrict__ vel, const float2* __restrict__ pr,
                     const float4* __restrict__ sums, uint32_t n, SimConst c, const float4* __restrict__ Xb,
@@ -103,8 +95,8 @@ __global__ void __launch_bounds__(kAdjBlock)
     }
     const float invb = dot3f(ab[0], ab[1], ab[2], t[0], t[1], t[2]);
     const float cvb = dot3f(tb[0], tb[1], tb[2], avs[0], avs[1], avs[2]);
-    st8(abrec + 2 * (size_t)i, make_float4(c.cp * tb[0], c.cp * tb[1], c.cp * tb[2], invb),
-        make_float4(c.cv * tb[0], c.cv * tb[1], c.cv * tb[2], cvb));
+    st8(abrec + 2 * (size_t)i, make_float4(c.cp * tb[0], c.cv * tb[0], c.cp * tb[1], c.cv * tb[1]),
+        make_float4(c.cp * tb[2], c.cv * tb[2], invb, cvb));
     xdir[i] = make_float4(xd[0], xd[1], xd[2], 0.f);
     vdir[i] = make_float4(vd[0], vd[1], vd[2], 0.f);
 }
@@ -131,124 +123,237 @@ __device__ __forceinline__ void eos_derivs(const SimConst& c, float rho, float& 
     dpdk = act ? dk : 0.f;
 }
 
+// The pair sums of P2 for particle k: x_bar and v_bar of the force terms in
+// both orientations, p_bar and inv_bar.
+struct AdjSums {
+    float xb[3] = {0.f, 0.f, 0.f}, vb[3] = {0.f, 0.f, 0.f}, pb = 0.f, inv = 0.f;
+};
+// What P2 knows of a particle: (x, vx) .. (z, vz), (p, 1/rho), and P1's
+// (apb, avb) of the axes, (inv_bar, cv_bar).
+struct AdjRec {
+    PairRec s, a;
+};
+__device__ __forceinline__ void ld_adj(const float4* __restrict__ pv, const float4* __restrict__ ab, uint32_t j,
+                                       AdjRec& r) {
+    ld_rec<true>(pv + 2 * (size_t)j, r.s);
+    ld_rec<true>(ab + 2 * (size_t)j, r.a);
+}
+
+// Terms of neighbour j (not k itself), with the compiler's root and divisions.
+__device__ __forceinline__ void adj_pair(float h, const AdjRec& k, const AdjRec& j, AdjSums& o) {
+    const float2 ek[3] = {unpack(k.s.x), unpack(k.s.y), unpack(k.s.z)}, ck[3] = {unpack(k.a.x), unpack(k.a.y), unpack(k.a.z)};
+    const float2 ej[3] = {unpack(j.s.x), unpack(j.s.y), unpack(j.s.z)}, cj[3] = {unpack(j.a.x), unpack(j.a.y), unpack(j.a.z)};
+    const float pk = unpack(k.s.pw).x, invk = unpack(k.s.pw).y, pj = unpack(j.s.pw).x, invj = unpack(j.s.pw).y;
+    const float d0 = ek[0].x - ej[0].x, d1 = ek[1].x - ej[1].x, d2 = ek[2].x - ej[2].x;
+    const float r2 = fmaf(d2, d2, fmaf(d1, d1, d0 * d0));
+    const float r = sqrtf(r2);
+    const float hr = h - r;
+    const float dv0 = ej[0].y - ek[0].y, dv1 = ej[1].y - ek[1].y, dv2 = ej[2].y - ek[2].y;
+    const float ps = pk + pj;
+    // orientation A: k is i, j the neighbour
+    const float wkj = hr * invj;
+#pragma unroll
+    for (int q = 0; q < 3; ++q) o.vb[q] = fmaf(-wkj, ck[q].y, o.vb[q]);
+    float wb = dot3f(ck[0].y, ck[1].y, ck[2].y, dv0, dv1, dv2);
+    float rb = 0.f;
+    // orientation B: j is i, k the neighbour
+    const float wjk = hr * invk;
+#pragma unroll
+    for (int q = 0; q < 3; ++q) o.vb[q] = fmaf(wjk, cj[q].y, o.vb[q]);
+    float wb2 = -dot3f(cj[0].y, cj[1].y, cj[2].y, dv0, dv1, dv2);
+    float rb2 = 0.f;
+    if (r > 0.f) {
+        const float q = hr / r;
+        const float S = (ps * wkj) * q;
+        const float Sb = dot3f(ck[0].x, ck[1].x, ck[2].x, d0, d1, d2);
+#pragma unroll
+        for (int x = 0; x < 3; ++x) o.xb[x] = fmaf(S, ck[x].x, o.xb[x]);
+        o.pb = fmaf(Sb, wkj * q, o.pb);
+        wb = fmaf(Sb, ps * q, wb);
+        const float qb = Sb * (ps * wkj);
+        rb = -((qb * h) / r2);
+        const float S2 = (ps * wjk) * q;
+        const float Sb2 = -dot3f(cj[0].x, cj[1].x, cj[2].x, d0, d1, d2);
+#pragma unroll
+        for (int x = 0; x < 3; ++x) o.xb[x] = fmaf(-S2, cj[x].x, o.xb[x]);
+        o.pb = fmaf(Sb2, wjk * q, o.pb);
+        wb2 = fmaf(Sb2, ps * q, wb2);
+        const float qb2 = Sb2 * (ps * wjk);
+        rb2 = -((qb2 * h) / r2);
+    }
+    rb = fmaf(-wb, invj, rb);
+    o.inv = fmaf(wb2, hr, o.inv);
+    rb2 = fmaf(-wb2, invk, rb2);
+    if (r > 0.f) {
+        const float g = (rb + rb2) / r;
+        o.xb[0] = fmaf(g, d0, o.xb[0]);
+        o.xb[1] = fmaf(g, d1, o.xb[1]);
+        o.xb[2] = fmaf(g, d2, o.xb[2]);
+    }
+}
+
+// The same of two neighbours a and b at once (`va`, `vb` clear: none, its
+// terms are zeros), a's added before b's, without the compiler's root and
+// divisions (see root_quotient): the packed halves are the position and the
+// velocity side of one neighbour in the differences, dot products and sums,
+// and the two neighbours in between.  Signs differ from adj_pair's where that
+// saves an operation; every rounding is the same.
+constexpr float kAdjTiny = 7.8886091e-31f;  // 2^-100: quotients of smaller numerators go to adj_pair
+constexpr float kAdjHMax = 1024.f;
+struct AdjPairSums {
+    F2 x, y, z;              // (x_bar, v_bar)
+    float pb = 0.f, inv = 0.f;
+    float nearest = 1.f;     // smallest r^2 so far
+    uint32_t tiny = ~0u;     // smallest 2 bits(|numerator|) - 1 so far (numerators that are zero pass)
+};
+__device__ __forceinline__ F2 quotient2(F2 num, F2 minus_den, F2 recip) {
+    const F2 q0 = mul2(num, recip);
+    return fma2(fma2(minus_den, q0, num), recip, q0);
+}
+__device__ __forceinline__ void adj_pair2(float h, const F2 k[3], float pk, F2 invk, const PairRec& ck, const AdjRec& a,
+                                          const AdjRec& b, bool va, bool vb, AdjPairSums& o) {
+    const F2 flip = f2(-1.f, 1.f), bias = f2(2.8421709e-14f, 2.8421709e-14f), one = f2(1.f, 1.f);
+    // (xk - xj, vj - vk); k holds (xk, -vk)
+    const F2 ax = fma2(a.s.x, flip, k[0]), ay = fma2(a.s.y, flip, k[1]), az = fma2(a.s.z, flip, k[2]);
+    const F2 bx = fma2(b.s.x, flip, k[0]), by = fma2(b.s.y, flip, k[1]), bz = fma2(b.s.z, flip, k[2]);
+    const float ra = va ? square3(ax, ay, az) : 1.f, rb = vb ? square3(bx, by, bz) : 1.f;
+    o.nearest = fminf(o.nearest, fminf(ra, rb));
+    const F2 n2 = f2(-ra, -rb), y0 = f2(rsqrt_approx(ra), rsqrt_approx(rb));
+    const F2 ns = mul2(n2, y0);
+    const F2 nr = fma2(fma2(ns, ns, n2), mul2(y0, f2(0.5f, 0.5f)), ns);  // -r
+    const F2 y = fma2(add2(fma2(nr, y0, one), bias), y0, y0);            // 1 / r
+    const F2 z0 = mul2(y0, y0);
+    const F2 y2 = fma2(add2(fma2(n2, z0, one), bias), z0, z0);           // 1 / r^2
+    const float2 hr1 = unpack(add2(f2(h, h), nr));
+    const F2 hr = f2(va ? hr1.x : 0.f, vb ? hr1.y : 0.f);  // zero weights where there is no neighbour
+    const F2 q = quotient2(hr, nr, y);
+    const float2 pa = unpack(a.s.pw), pb = unpack(b.s.pw);
+    const F2 ps = f2(pk + pa.x, pk + pb.x), inv = f2(pa.y, pb.y);
+    const F2 wkj = mul2(hr, inv), wjk = mul2(hr, invk);
+    // (Sb, wb) and minus (Sb2, wb2) of each neighbour
+    const float2 fa = unpack(fma2(ck.z, az, fma2(ck.y, ay, mul2(ck.x, ax))));
+    const float2 fb = unpack(fma2(ck.z, bz, fma2(ck.y, by, mul2(ck.x, bx))));
+    const float2 ga = unpack(fma2(a.a.z, az, fma2(a.a.y, ay, mul2(a.a.x, ax))));
+    const float2 gb = unpack(fma2(b.a.z, bz, fma2(b.a.y, by, mul2(b.a.x, bx))));
+    const F2 Sb = f2(fa.x, fb.x), nSb2 = f2(ga.x, gb.x);
+    const F2 t1 = mul2(ps, wkj), t2 = mul2(ps, wjk), pq = mul2(ps, q);
+    const F2 wb = fma2(Sb, pq, f2(fa.y, fb.y)), nwb2 = fma2(nSb2, pq, f2(ga.y, gb.y));
+    const F2 hh = f2(h, h);
+    const F2 n1 = mul2(mul2(Sb, t1), hh), m1 = mul2(mul2(nSb2, t2), hh);
+    const F2 nrb = fma2(wb, inv, quotient2(n1, n2, y2));    // minus rb
+    const F2 rb2 = fma2(nwb2, invk, quotient2(m1, n2, y2));
+    const F2 gn = fma2(nrb, f2(-1.f, -1.f), rb2);           // rb + rb2
+    const float2 g = unpack(quotient2(gn, nr, y));
+    auto seen = [&](F2 v) {
+        const float2 u = unpack(v);
+        o.tiny = min(o.tiny, min(2u * __float_as_uint(u.x) - 1u, 2u * __float_as_uint(u.y) - 1u));
+    };
+    seen(n1);
+    seen(m1);
+    seen(gn);
+    const float2 S = unpack(mul2(t1, q)), S2 = unpack(mul2(t2, q)), w1 = unpack(wkj), w2 = unpack(wjk);
+    const float2 kq = unpack(mul2(wkj, q)), jq = unpack(mul2(wjk, q)), hru = unpack(hr), nw = unpack(nwb2);
+    auto add = [&](F2 ex, F2 ey, F2 ez, const PairRec& cj, float s, float s2, float wk, float wj, float gg) {
+        const F2 u = f2(s, -wk), v = f2(-s2, wj);
+        auto axis = [&](F2& sum, F2 c, F2 cn, F2 e) {
+            const float2 t = unpack(fma2(v, cn, fma2(u, c, sum)));
+            sum = f2(fmaf(gg, unpack(e).x, t.x), t.y);
+        };
+        axis(o.x, ck.x, cj.x, ex);
+        axis(o.y, ck.y, cj.y, ey);
+        axis(o.z, ck.z, cj.z, ez);
+    };
+    add(ax, ay, az, a.a, S.x, S2.x, w1.x, w2.x, g.x);
+    o.pb = fmaf(-ga.x, jq.x, fmaf(fa.x, kq.x, o.pb));
+    o.inv = fmaf(-nw.x, hru.x, o.inv);
+    add(bx, by, bz, b.a, S.y, S2.y, w1.y, w2.y, g.y);
+    o.pb = fmaf(-gb.x, jq.y, fmaf(fb.x, kq.y, o.pb));
+    o.inv = fmaf(-nw.y, hru.y, o.inv);
+}
+
 // P2: force pair terms of every pair in both orientations, then the density
 // adjoint of the particle.  Outputs xrb = (x, y, z, rho_bar), P4's gather
 // record, xf = (force x_bar, k_bar) and vf.
 // A neighbour is two 32-byte records, each one 256-bit load: the step's
-// gather record and P1's (apb | avb).
+// gather record and P1's.
+// 65,536 particles are 13.5 warps per SM, so the pass takes as long as a
+// thread's chain: two neighbours share each of its steps (adj_pair2, half the
+// instructions of adj_pair, none of its branches), and the next two's records
+// are on their way meanwhile.  47 -> 31 us by the first, -> 24 us by the
+// second (65,536 disordered particles), 84 -> 43 us at 150,000; blocks of 64
+// threads spread the warps evenly (32: 26 us).
 template <int kReach>
-__global__ void __launch_bounds__(kAdjBlock)
-    k_adj_forces(const float4* __restrict__ pos, const float4* __restrict__ pv, const float2* __restrict__ pr,
-                 const float* __restrict__ rho, const uint32_t* __restrict__ cs, const uint32_t* __restrict__ nbr,
-                 const uint32_t* __restrict__ cnt, uint32_t n, SimConst c, const float4* __restrict__ ab,
-                 float4* __restrict__ xrb, float4* __restrict__ xf, float4* __restrict__ vf) {
-    const uint32_t k = blockIdx.x * kAdjBlock + threadIdx.x;
+__global__ void __launch_bounds__(kAdjForceBlock)
+    k_adj_forces(const float4* __restrict__ pos, const float4* __restrict__ pv, const float* __restrict__ rho,
+                 const uint32_t* __restrict__ cs, const uint32_t* __restrict__ nbr, const uint32_t* __restrict__ cnt,
+                 uint32_t n, SimConst c, const float4* __restrict__ ab, float4* __restrict__ xrb,
+                 float4* __restrict__ xf, float4* __restrict__ vf) {
+    const uint32_t k = blockIdx.x * kAdjForceBlock + threadIdx.x;
     if (k >= n) return;
-    float4 xk, vk, apbk, avbk;
-    ld_state(pv + 2 * (size_t)k, xk, vk);
-    ld8(ab + 2 * (size_t)k, apbk, avbk);
-    const float2 prk = pr[k];
-    const float pk = prk.x, invk = prk.y;
-    float pb = 0.f, invacc = 0.f;
-    float xb0 = 0.f, xb1 = 0.f, xb2 = 0.f, vb0 = 0.f, vb1 = 0.f, vb2 = 0.f;
-    auto pair = [&](const float4& xj, const float4& vj, const float4& apbj, const float4& avbj) {
-        const float d0 = xk.x - xj.x, d1 = xk.y - xj.y, d2 = xk.z - xj.z;
-        const float r2 = fmaf(d2, d2, fmaf(d1, d1, d0 * d0));
-        const float r = sqrtf(r2);
-        const float hr = c.h - r;
-        const float pj = xj.w, invj = vj.w;
-        const float dv0 = vj.x - vk.x, dv1 = vj.y - vk.y, dv2 = vj.z - vk.z;
-        const float ps = pk + pj;
-        // orientation A: k is i, j the neighbour
-        const float wkj = hr * invj;
-        vb0 = fmaf(-wkj, avbk.x, vb0);
-        vb1 = fmaf(-wkj, avbk.y, vb1);
-        vb2 = fmaf(-wkj, avbk.z, vb2);
-        float wb = dot3f(avbk.x, avbk.y, avbk.z, dv0, dv1, dv2);
-        float rb = 0.f;
-        // orientation B: j is i, k the neighbour
-        const float wjk = hr * invk;
-        vb0 = fmaf(wjk, avbj.x, vb0);
-        vb1 = fmaf(wjk, avbj.y, vb1);
-        vb2 = fmaf(wjk, avbj.z, vb2);
-        float wb2 = -dot3f(avbj.x, avbj.y, avbj.z, dv0, dv1, dv2);
-        float rb2 = 0.f;
-        if (r > 0.f) {
-            const float q = hr / r;
-            const float S = (ps * wkj) * q;
-            const float Sb = dot3f(apbk.x, apbk.y, apbk.z, d0, d1, d2);
-            xb0 = fmaf(S, apbk.x, xb0);
-            xb1 = fmaf(S, apbk.y, xb1);
-            xb2 = fmaf(S, apbk.z, xb2);
-            pb = fmaf(Sb, wkj * q, pb);
-            wb = fmaf(Sb, ps * q, wb);
-            const float qb = Sb * (ps * wkj);
-            rb = -((qb * c.h) / r2);
-            const float S2 = (ps * wjk) * q;
-            const float Sb2 = -dot3f(apbj.x, apbj.y, apbj.z, d0, d1, d2);
-            xb0 = fmaf(-S2, apbj.x, xb0);
-            xb1 = fmaf(-S2, apbj.y, xb1);
-            xb2 = fmaf(-S2, apbj.z, xb2);
-            pb = fmaf(Sb2, wjk * q, pb);
-            wb2 = fmaf(Sb2, ps * q, wb2);
-            const float qb2 = Sb2 * (ps * wjk);
-            rb2 = -((qb2 * c.h) / r2);
-        }
-        rb = fmaf(-wb, invj, rb);
-        invacc = fmaf(wb2, hr, invacc);
-        rb2 = fmaf(-wb2, invk, rb2);
-        if (r > 0.f) {
-            const float g = (rb + rb2) / r;
-            xb0 = fmaf(g, d0, xb0);
-            xb1 = fmaf(g, d1, xb1);
-            xb2 = fmaf(g, d2, xb2);
-        }
-    };
     const uint32_t m = __ldg(cnt + k);
+    const uint32_t* lst = nbr + nbr_index(k, 0);  // slot s at lst[s * kNbTile]
+    uint32_t ea = __ldg(lst), eb = __ldg(lst + kNbTile);
+    AdjRec me;
+    ld_adj(pv, ab, k, me);
+    const float2 x = unpack(me.s.x), y = unpack(me.s.y), z = unpack(me.s.z), pw = unpack(me.s.pw);
+    AdjSums o;
+    bool summed = false;
     if (m <= (uint32_t)kNbCap) {
-        // The next neighbour's records and the index after it are in flight
-        // while a neighbour is processed.  The list holds the particle itself
-        // (skipped); slots past the count hold stale values, never used.
-        const uint32_t* lst = nbr + nbr_index(k, 0);  // slot s at lst[s * kNbTile]
-        uint32_t jc = checked_index(__ldg(lst), n), jn = __ldg(lst + kNbTile);
-        float4 nx, nv, na, nb;
-        if (m) {
-            ld_state(pv + 2 * (size_t)jc, nx, nv);
-            ld8(ab + 2 * (size_t)jc, na, nb);
+        const F2 mine[3] = {f2(x.x, -x.y), f2(y.x, -y.y), f2(z.x, -z.y)};
+        AdjPairSums p;
+        p.x = p.y = p.z = f2(0.f, 0.f);
+        // The next two neighbours' records and the entries after them are on
+        // their way while two are processed.  The list holds the particle
+        // itself (no terms); slots past the count hold stale values, never used.
+        uint32_t ja = m ? checked_index(ea, n) : k, jb = 1 < m ? checked_index(eb, n) : k;
+        AdjRec a, b;
+        ld_adj(pv, ab, ja, a);
+        ld_adj(pv, ab, jb, b);
+        lst += 2 * kNbTile;
+        ea = __ldg(lst);
+        eb = __ldg(lst + kNbTile);
+#pragma unroll 1
+        for (uint32_t s = 0; s < m; s += 2) {
+            const bool va = ja != k, vb = jb != k;
+            ja = s + 2 < m ? checked_index(ea, n) : k;
+            jb = s + 3 < m ? checked_index(eb, n) : k;
+            AdjRec na, nb;
+            ld_adj(pv, ab, ja, na);
+            ld_adj(pv, ab, jb, nb);
+            lst += s + 4 < m ? 2 * kNbTile : 0;
+            ea = __ldg(lst);
+            eb = __ldg(lst + kNbTile);
+            adj_pair2(c.h, mine, pw.x, f2(pw.y, pw.y), me.a, a, b, va, vb, p);
+            a = na;
+            b = nb;
         }
-        for (uint32_t s = 0; s < m; ++s) {
-            const uint32_t j = jc;
-            const float4 xj = nx, vj = nv, apbj = na, avbj = nb;
-            if (s + 1 < m) {
-                jc = checked_index(jn, n);
-                jn = __ldg(lst + (size_t)min(s + 2, (uint32_t)kNbCap - 1) * kNbTile);
-                ld_state(pv + 2 * (size_t)jc, nx, nv);
-                ld8(ab + 2 * (size_t)jc, na, nb);
-            }
-            if (j != k) pair(xj, vj, apbj, avbj);
-        }
-    } else {
-        for_candidates<kReach>(c, cs, pos, n, xk.x, xk.y, xk.z, [&](uint32_t j, const float4& xp) {
+        const float2 sx = unpack(p.x), sy = unpack(p.y), sz = unpack(p.z);
+        o = AdjSums{{sx.x, sy.x, sz.x}, {sx.y, sy.y, sz.y}, p.pb, p.inv};
+        summed = c.h >= kFastHMin && c.h <= kAdjHMax && p.nearest >= kFastR2Min &&
+                 p.tiny >= 2u * __float_as_uint(kAdjTiny) - 1u && isfinite(sx.x + sy.x + sz.x);
+    }
+    if (!summed) {
+        o = AdjSums{};
+        for_candidates_rolled<kReach>(c, cs, pos, n, x.x, y.x, z.x, [&](uint32_t j, const float4& xp) {
             if (j == k) return;
-            const float dx = xk.x - xp.x, dy = xk.y - xp.y, dz = xk.z - xp.z;
+            const float dx = x.x - xp.x, dy = y.x - xp.y, dz = z.x - xp.z;
             if (!(fmaf(dz, dz, fmaf(dy, dy, dx * dx)) < c.h2)) return;
-            float4 xj, vj, apbj, avbj;
-            ld_state(pv + 2 * (size_t)j, xj, vj);
-            ld8(ab + 2 * (size_t)j, apbj, avbj);
-            pair(xj, vj, apbj, avbj);
+            AdjRec r;
+            ld_adj(pv, ab, j, r);
+            adj_pair(c.h, me, r, o);
         });
     }
-    const float ib = apbk.w + invacc;
+    const float ib = unpack(me.a.pw).x + o.inv;
     float dpdrho, dpdk;
     eos_derivs(c, rho[k], dpdrho, dpdk);
-    xrb[k] = make_float4(xk.x, xk.y, xk.z, fmaf(pb, dpdrho, -((ib * invk) * invk)));
-    xf[k] = make_float4(xb0, xb1, xb2, pb * dpdk);
-    vf[k] = make_float4(vb0, vb1, vb2, 0.f);
+    xrb[k] = make_float4(x.x, y.x, z.x, fmaf(o.pb, dpdrho, -((ib * pw.y) * pw.y)));
+    xf[k] = make_float4(o.xb[0], o.xb[1], o.xb[2], o.pb * dpdk);
+    vf[k] = make_float4(o.vb[0], o.vb[1], o.vb[2], 0.f);
 }
 
 // P4: poly6 density terms onto positions; the step's input adjoints are
 // written back by particle id.
-// Also reduces the step's scalar adjoints (cv_bar in avb.w of the ab record, k_bar in xf.w) per
+// Also reduces the step's scalar adjoints (cv_bar in the ab record's last word, k_bar in xf.w) per
 // block, in thread order, into partial[blockIdx.x].
 template <int kReach>
 __global__ void __launch_bounds__(kAdjBlock)
@@ -453,8 +558,8 @@ void launch_adjoint_pass(uint32_t pass, const AdjointStep& st, const SimConst& c
     with_reach(c.reach, [&](auto R) {
         constexpr int K = decltype(R)::value;
         if (pass == 1)
-            k_adj_forces<K><<<g, kAdjBlock, 0, s>>>(st.pos, st.pv, st.pr, st.rho, st.cs, st.nbr, st.cnt, n, c, w.ab,
-                                                    w.xrb, w.xf, w.vf);
+            k_adj_forces<K><<<grid_for(n, kAdjForceBlock), kAdjForceBlock, 0, s>>>(
+                st.pos, st.pv, st.rho, st.cs, st.nbr, st.cnt, n, c, w.ab, w.xrb, w.xf, w.vf);
         else if (pass == 2)
             k_adj_density<K><<<g, kAdjBlock, 0, s>>>(st.pos, st.cs, st.nbr, st.cnt, n, c, m6cd, w.xrb, w.xdir, w.vdir,
                                                      w.xf, w.vf, w.ab, w.Xb, w.Vb, partial);

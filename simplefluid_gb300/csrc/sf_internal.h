@@ -236,7 +236,7 @@ struct AdjointStep {
 struct AdjointWork {
     float4* Xb = nullptr;
     float4* Vb = nullptr;
-    float4* ab = nullptr;  // 2 per particle (32 bytes): apb = (cp tb, inv_bar), avb = (cv tb, cv_bar)
+    float4* ab = nullptr;  // 2 per particle (32 bytes): (apb, avb) = (cp tb, cv tb) of the axes, (inv_bar, cv_bar)
     float4* xdir = nullptr;
     float4* vdir = nullptr;
     float4* xf = nullptr;

@@ -101,3 +101,27 @@ def test_root_and_quotient_at_every_scale(h):
         got = run(prm, pos, vel, tune)
         for k in (0, 1, 2, 4, 5):
             np.testing.assert_array_equal(got[k], want[k])
+
+
+@pytest.mark.parametrize("seed_scale", [1.0, 1e-20, 1e-33, 1e-38])
+@pytest.mark.parametrize("h", [0.04, 2.0 ** -5, 2048.0])
+def test_adjoint_pairs_equal_oracle(oracle, h, seed_scale):
+    """The adjoint's paired force terms: kernel radii in and out of their range, adjoints down to numbers whose
+    quotients underflow (most particles have none), coincident and nearly coincident particles."""
+    n = 700
+    pos, vel = block(n, 5)
+    pos = (pos * (h / 0.04)).astype(np.float32)
+    pos[10:12] = pos[9]
+    pos[20] = pos[21] + np.float32(1e-6 * h)
+    vel = (vel * h).astype(np.float32)
+    prm = params_16k(kernelRadius=h, particleRadius=h / 4, boxMax=(25 * h,) * 3, timeStep=1e-6)
+    rng = np.random.default_rng(3)
+    gx = np.zeros((n, 3), np.float32)
+    gx[::50] = (seed_scale * rng.normal(size=gx[::50].shape)).astype(np.float32)
+    with SPHSolver(prm) as s:
+        s.setParticles(pos, vel)
+        s.forward(3, 2)
+        dx0, dv0, _, _ = s.adjoint(gx)
+    want = oracle.adjoint(prm.to_c(), pos, vel, 3, gx, ckpt=2, dtype=np.float32)
+    np.testing.assert_array_equal(dx0, want[0])
+    np.testing.assert_array_equal(dv0, want[1])
