@@ -190,7 +190,8 @@ extern "C" {
 
 SF_API sf_status sf_forward(sf_ctx* ctx, uint32_t nsteps, uint32_t ckpt_every) {
     SF_RANGE("sf_forward");
-    SF_TRY(sf_make_ready(ctx));
+    SF_TRY(need_sorted(ctx));
+    SF_TRY(set_device(ctx));
     if (ctx->c.adaptive) return fail(SF_ERR_INVALID_ARGUMENT, "differentiation needs a fixed time step");
     if (ckpt_every == 0) return fail(SF_ERR_INVALID_ARGUMENT, "ckpt_every must be > 0");
     if (!ctx->traj) ctx->traj = new sf::Trajectory();
@@ -206,14 +207,13 @@ SF_API sf_status sf_forward(sf_ctx* ctx, uint32_t nsteps, uint32_t ckpt_every) {
         for (auto& p : t->ck) SF_ALLOC_TRAJ(p, 2 * (size_t)d.cap * sizeof(float4));
     }
     t->valid = false;
-    for (uint32_t s = 0; s < nsteps; ++s) {
-        if (s % ckpt_every == 0) {
-            float4* c = t->ck[s / ckpt_every];
-            SF_CUDA(cudaMemcpyAsync(c, d.pos, (size_t)d.n * sizeof(float4), cudaMemcpyDeviceToDevice, ctx->stream));
-            SF_CUDA(cudaMemcpyAsync(c + d.n, d.vel, (size_t)d.n * sizeof(float4), cudaMemcpyDeviceToDevice,
-                                    ctx->stream));
-        }
-        SF_CUDA(cudaGraphLaunch(ctx->step_graph, ctx->stream));
+    for (uint32_t s = 0; s < nsteps;) {
+        float4* c = t->ck[s / ckpt_every];
+        SF_CUDA(cudaMemcpyAsync(c, d.pos, (size_t)d.n * sizeof(float4), cudaMemcpyDeviceToDevice, ctx->stream));
+        SF_CUDA(cudaMemcpyAsync(c + d.n, d.vel, (size_t)d.n * sizeof(float4), cudaMemcpyDeviceToDevice, ctx->stream));
+        const uint32_t len = std::min(ckpt_every, nsteps - s);
+        SF_TRY(launch_steps(ctx, len));
+        s += len;
     }
     t->nsteps = nsteps;
     t->ckpt = ckpt_every;

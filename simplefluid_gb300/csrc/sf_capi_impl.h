@@ -67,7 +67,9 @@ struct sf_ctx {
     int host_direct = -1;
     uint32_t* d_report = nullptr;  // sf_check_state counters
     bool tune_explicit = false;    // sf_set_tuning was called: keep its choices
-    cudaGraphExec_t step_graph = nullptr;
+    cudaGraphExec_t step_graph = nullptr;  // one sub-step
+    cudaGraphExec_t run_graph = nullptr;   // kRunSteps sub-steps
+    bool stepped = false;                  // a call stepped since the graphs were last dropped
     bool sorted = false;  // particles uploaded and cell-sorted
     float* h_stage = nullptr;  // pinned staging for pageable caller buffers
     size_t h_stage_bytes = 0;
@@ -154,7 +156,9 @@ void release_ctx(sf_ctx* ctx);
 sf_status sort_uploaded(sf_ctx* ctx, const float* pos3, const float* vel3);
 sf_status upload_overlapped(sf_ctx* ctx, const float* pos_xyz, const float* vel_xyz);
 void enqueue_full_step(sf_ctx* ctx);
-sf_status capture_step(sf_ctx* ctx);
+// A graph of `nsteps` sub-steps; and nsteps sub-steps queued on the stream.
+sf_status capture_steps(sf_ctx* ctx, uint32_t nsteps, cudaGraphExec_t* out);
+sf_status launch_steps(sf_ctx* ctx, uint32_t nsteps);
 void drop_graph(sf_ctx* ctx);
 // Kernel choices by particle count, unless the caller set them explicitly.
 void apply_size_defaults(sf_ctx* ctx);
