@@ -275,8 +275,7 @@ sf_status check_launch(const char* what) {
 // sort it into the cell order.
 sf_status sort_uploaded(sf_ctx* ctx, const float* pos3, const float* vel3) {
     sf::DeviceState& d = ctx->d;
-    sf::launch_load_aos(pos3, vel3, d.n, d.pos2, d.vel2, ctx->stream);
-    sf::launch_hash_count(d, d.pos2, d.n, ctx->c, d.counts, d.key_slot, ctx->stream);
+    sf::launch_load_hash(d, pos3, vel3, d.vel2, ctx->c, ctx->stream);
     sf::enqueue_sort_tail(d, ctx->stream);
     if (ctx->frame && ctx->c.adaptive) sf::launch_init_maxima(d.vel, d.n, ctx->frame, ctx->stream);
     SF_TRY(check_launch("initial sort"));
@@ -309,8 +308,7 @@ sf_status upload_overlapped(sf_ctx* ctx, const float* pos_xyz, const float* vel_
     SF_CUDA(cudaEventRecord(ctx->ev_in, ctx->aux));
     sf::launch_load_vel(io_vel, d.n, d.vel2, ctx->aux);
     SF_CUDA(cudaEventRecord(ctx->ev_vel, ctx->aux));
-    sf::launch_load_pos(io_pos, d.n, d.pos2, ctx->stream);
-    sf::launch_hash_count(d, d.pos2, d.n, ctx->c, d.counts, d.key_slot, ctx->stream);
+    sf::launch_load_hash(d, io_pos, nullptr, nullptr, ctx->c, ctx->stream);
     sf::enqueue_sort_tail(d, ctx->stream, ctx->ev_vel);
     if (ctx->frame && ctx->c.adaptive) sf::launch_init_maxima(d.vel, d.n, ctx->frame, ctx->stream);
     SF_TRY(check_launch("initial sort"));

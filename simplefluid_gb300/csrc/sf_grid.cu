@@ -16,24 +16,24 @@ namespace sf {
 namespace {
 
 // ---------------------------------------------------------------- state IO
-__global__ void k_load_aos(const float* __restrict__ pos3, const float* __restrict__ vel3, uint32_t n,
-                           float4* __restrict__ pos, float4* __restrict__ vel) {
-    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    pos[i] = make_float4(pos3[3 * (size_t)i], pos3[3 * (size_t)i + 1], pos3[3 * (size_t)i + 2], __uint_as_float(i));
-    if (vel3)
-        vel[i] = make_float4(vel3[3 * (size_t)i], vel3[3 * (size_t)i + 1], vel3[3 * (size_t)i + 2], 0.f);
-    else
-        vel[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+// A full warp's 32 consecutive AoS entries written as three contiguous runs of
+// 128 bytes, through `row` (96 floats of shared memory of the warp's own).  The
+// three runs of stride 12 that the lanes hold make three partial writes of
+// every sector, and over the CPU-GPU link each costs a transfer: reading back
+// 1,048,576 particles 260 -> 177 us.  (Loads gain nothing from the same: the
+// sectors stay in L1 between the three.)
+__device__ __forceinline__ void store_row(float* __restrict__ first, float* row, const float4& v) {
+    const unsigned lane = threadIdx.x & 31;
+    __syncwarp();
+    row[3 * lane] = v.x;
+    row[3 * lane + 1] = v.y;
+    row[3 * lane + 2] = v.z;
+    __syncwarp();
+#pragma unroll
+    for (int k = 0; k < 3; ++k) first[32 * k + lane] = row[32 * k + lane];
 }
 
-// The two halves of k_load_aos, for uploads whose velocities arrive later.
-__global__ void k_load_pos(const float* __restrict__ pos3, uint32_t n, float4* __restrict__ pos) {
-    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    pos[i] = make_float4(pos3[3 * (size_t)i], pos3[3 * (size_t)i + 1], pos3[3 * (size_t)i + 2], __uint_as_float(i));
-}
-
+// Velocities that arrive after k_load_hash took the positions.
 __global__ void k_load_vel(const float* __restrict__ vel3, uint32_t n, float4* __restrict__ vel) {
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
@@ -67,6 +67,7 @@ __global__ void k_store_sorted(const float4* __restrict__ pos, const float4* __r
 
 __global__ void k_store_aos(const float4* __restrict__ pos, const float4* __restrict__ vel, uint32_t n,
                             float* __restrict__ pos3, float* __restrict__ vel3) {
+    grid_dependency_wait();
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     const float4 p = pos[i];
@@ -87,6 +88,8 @@ __global__ void k_store_aos(const float4* __restrict__ pos, const float4* __rest
 
 // Sorted slot of every caller index.
 __global__ void k_slot_of_caller(const float4* __restrict__ pos, uint32_t n, uint32_t* __restrict__ slot) {
+    grid_dependency_wait();
+    allow_dependents();
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     const uint32_t id = __float_as_uint(pos[i].w);
@@ -94,15 +97,23 @@ __global__ void k_slot_of_caller(const float4* __restrict__ pos, uint32_t n, uin
 }
 
 // Caller-order AoS state gathered through the slot map: consecutive threads
-// write consecutive particles, so the stores stay coalesced when the arrays
-// are host memory that the kernel writes over the CPU-GPU link.
+// write consecutive particles, and full warps whole rows, since the arrays are
+// host memory that the kernel writes over the CPU-GPU link.
 __global__ void k_store_caller_order(const float4* __restrict__ pos, const float4* __restrict__ vel,
                                      const uint32_t* __restrict__ slot, uint32_t n, float* __restrict__ pos3,
                                      float* __restrict__ vel3) {
+    grid_dependency_wait();
     const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= n) return;
-    const uint32_t i = slot[t];
-    if (i >= n) return;  // never for a consistent state
+    const uint32_t i = t < n ? slot[t] : n;
+    __shared__ float rows[kBlock * 3];
+    if (__all_sync(0xffffffffu, i < n)) {
+        float* const row = rows + (threadIdx.x & ~31u) * 3;
+        const size_t first = 3 * (size_t)(t & ~31u);
+        if (pos3) store_row(pos3 + first, row, pos[i]);
+        if (vel3) store_row(vel3 + first, row, vel[i]);
+        return;
+    }
+    if (i >= n) return;  // past the end (or, never for a consistent state, no such slot)
     if (pos3) {
         const float4 p = pos[i];
         pos3[3 * (size_t)t] = p.x;
@@ -118,13 +129,38 @@ __global__ void k_store_caller_order(const float4* __restrict__ pos, const float
 }
 
 // ---------------------------------------------------------------- hashing
-// Histogram of an uploaded (not cell-sorted) state.  Its lanes hit scattered
-// scan tiles, so the tile totals come from a separate reduction instead of
-// per-particle tile atomics.
+// A caller-order state loaded and counted in one pass (two passes and a plain
+// launch between them before: upload and sort of 16,000 particles 18.3 -> 13.8
+// us, of 1,048,576 63.7 -> 56.8).  Bound by the launches below 100,000
+// particles, by the histogram's atomics above.
+template <bool kBatched>
+__global__ void k_load_hash(const float* __restrict__ pos3, const float* __restrict__ vel3, uint32_t n, SimConst c0,
+                            const SimConst* __restrict__ table, const uint32_t* __restrict__ scene_off,
+                            uint32_t nscenes, float4* __restrict__ pos, float4* __restrict__ vel,
+                            uint32_t* __restrict__ counts, uint32_t* __restrict__ tile_sums,
+                            uint2* __restrict__ key_slot) {
+    allow_dependents();
+    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= n) return;
+    const float x = pos3[3 * (size_t)i], y = pos3[3 * (size_t)i + 1], z = pos3[3 * (size_t)i + 2];
+    const SimConst c = const_of<kBatched>(c0, table, scene_off, nscenes, i);
+    const uint32_t key = cell_key(c, x, y, z);
+    pos[i] = make_float4(x, y, z, __uint_as_float(i));
+    if (vel) {
+        if (vel3)
+            vel[i] = make_float4(vel3[3 * (size_t)i], vel3[3 * (size_t)i + 1], vel3[3 * (size_t)i + 2], 0.f);
+        else
+            vel[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+    }
+    key_slot[i] = make_uint2(key, count_in_cell(key, counts, tile_sums));
+}
+
+// Histogram of a loaded (not cell-sorted) state.
 template <bool kBatched>
 __global__ void k_hash_count(const float4* __restrict__ pos, uint32_t n, SimConst c0, const SimConst* __restrict__ table,
                              const uint32_t* __restrict__ scene_off, uint32_t nscenes, uint32_t* __restrict__ counts,
                              uint2* __restrict__ key_slot) {
+    allow_dependents();
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     const SimConst c = const_of<kBatched>(c0, table, scene_off, nscenes, i);
@@ -177,6 +213,8 @@ __device__ __forceinline__ uint32_t block_exclusive(uint32_t v, uint32_t* total)
 __global__ void __launch_bounds__(kScanThreads) k_tile_totals(const uint4* __restrict__ counts,
                                                               uint32_t* __restrict__ tile_sums) {
     __shared__ uint32_t total;
+    grid_dependency_wait();
+    allow_dependents();
     const uint4 q = counts[(size_t)blockIdx.x * kScanThreads + threadIdx.x];
     block_exclusive(q.x + q.y + q.z + q.w, &total);
     if (threadIdx.x == 0) tile_sums[blockIdx.x] = total;
@@ -417,12 +455,22 @@ void launch_check_state(const DeviceState& d, const SimConst& c, const uint32_t*
                                                                       nullptr, nullptr, 0, seen, report);
     k_check_ids<<<grid_for(d.n, kBlock), kBlock, 0, s>>>(seen, d.n, report);
 }
-void launch_load_aos(const float* pos3, const float* vel3, uint32_t n, float4* pos, float4* vel, cudaStream_t s) {
-    if (n) k_load_aos<<<grid_for(n, kBlock), kBlock, 0, s>>>(pos3, vel3, n, pos, vel);
+static void launch_tile_totals(const DeviceState& d, const uint32_t* counts, cudaStream_t s) {
+    launch_chained(k_tile_totals, d.ntiles, kScanThreads, s, reinterpret_cast<const uint4*>(counts), d.tile_sums);
 }
 
-void launch_load_pos(const float* pos3, uint32_t n, float4* pos, cudaStream_t s) {
-    if (n) k_load_pos<<<grid_for(n, kBlock), kBlock, 0, s>>>(pos3, n, pos);
+void launch_load_hash(const DeviceState& d, const float* pos3, const float* vel3, float4* vel, const SimConst& c,
+                      cudaStream_t s) {
+    const uint32_t n = d.n;
+    if (!n) return;
+    uint32_t* const tiles = n < kTileAtomics ? d.tile_sums : nullptr;
+    if (d.table)
+        k_load_hash<true><<<grid_for(n, kBlock), kBlock, 0, s>>>(pos3, vel3, n, c, d.table, d.scene_off, d.nscenes,
+                                                                 d.pos2, vel, d.counts, tiles, d.key_slot);
+    else
+        k_load_hash<false><<<grid_for(n, kBlock), kBlock, 0, s>>>(pos3, vel3, n, c, nullptr, nullptr, 0, d.pos2, vel,
+                                                                  d.counts, tiles, d.key_slot);
+    if (!tiles) launch_tile_totals(d, d.counts, s);
 }
 
 void launch_load_vel(const float* vel3, uint32_t n, float4* vel, cudaStream_t s) {
@@ -440,14 +488,14 @@ void launch_store_sorted(const float4* pos, const float4* vel, uint32_t n, float
 }
 
 void launch_store_aos(const float4* pos, const float4* vel, uint32_t n, float* pos3, float* vel3, cudaStream_t s) {
-    if (n) k_store_aos<<<grid_for(n, kBlock), kBlock, 0, s>>>(pos, vel, n, pos3, vel3);
+    if (n) launch_chained(k_store_aos, grid_for(n, kBlock), kBlock, s, pos, vel, n, pos3, vel3);
 }
 
 void launch_store_caller_order(const float4* pos, const float4* vel, uint32_t n, uint32_t* slot, float* pos3,
                                float* vel3, cudaStream_t s) {
     if (!n) return;
-    k_slot_of_caller<<<grid_for(n, kBlock), kBlock, 0, s>>>(pos, n, slot);
-    k_store_caller_order<<<grid_for(n, kBlock), kBlock, 0, s>>>(pos, vel, slot, n, pos3, vel3);
+    launch_chained(k_slot_of_caller, grid_for(n, kBlock), kBlock, s, pos, n, slot);
+    launch_chained(k_store_caller_order, grid_for(n, kBlock), kBlock, s, pos, vel, slot, n, pos3, vel3);
 }
 
 void launch_hash_count(const DeviceState& d, const float4* pos, uint32_t n, const SimConst& c, uint32_t* counts,
@@ -458,7 +506,7 @@ void launch_hash_count(const DeviceState& d, const float4* pos, uint32_t n, cons
                                                                   key_slot);
     else
         k_hash_count<false><<<grid_for(n, kBlock), kBlock, 0, s>>>(pos, n, c, nullptr, nullptr, 0, counts, key_slot);
-    k_tile_totals<<<d.ntiles, kScanThreads, 0, s>>>(reinterpret_cast<const uint4*>(counts), d.tile_sums);
+    launch_tile_totals(d, counts, s);
 }
 
 void launch_keys(const DeviceState& d, const float4* pos, uint32_t n, const SimConst& c, uint32_t* keys,
