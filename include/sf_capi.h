@@ -442,7 +442,7 @@ SF_API sf_status sf_batch_autotune(sf_batch* b, uint32_t trial_steps, sf_tuning*
  * caller's particle order; either output may be NULL, not both.  Work is
  * queued on `stream` (a cudaStream_t; NULL = default stream) and not waited
  * for.  Calls no allocator: the grid sort runs in one fixed static device
- * array (about 7.6 MB, held by every GPU that loads the library until exit),
+ * array (about 8.3 MB, held by every GPU that loads the library until exit),
  * which limits a call to 65,536 particles and 262,144 grid cells; larger
  * requests fail with SF_ERR_CAPACITY before any GPU work.  All calls share that
  * array: calls whose GPU work overlaps race, so serialise them on one stream.

@@ -105,7 +105,7 @@ __global__ void __launch_bounds__(kPBlock) k_batch_persistent(BatchStep a) {
             uint32_t v2 = 0u, a2 = 0u;
             force_one<1, 2, true, kReach, false, false>(i, a.pos, a.vel, a.pr, a.cell_start, a.nbr, a.nbr_count,
                                                         nullptr, a.pv, a.n, c, nullptr, nullptr, 0u, a.pos2, a.vel2,
-                                                        a.counts, nullptr, a.key_slot, nullptr, nullptr, nullptr, v2,
+                                                        a.counts, nullptr, nullptr, a.key_slot, nullptr, nullptr, nullptr, v2,
                                                         a2);
         }
         cluster_sync();

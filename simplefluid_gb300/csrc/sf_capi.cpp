@@ -139,10 +139,8 @@ void free_particles(sf::DeviceState& d) {
 }
 
 void free_grid(sf::DeviceState& d) {
-    if (d.counts) cudaFree(d.counts);
-    if (d.cell_start) cudaFree(d.cell_start);
-    if (d.tile_sums) cudaFree(d.tile_sums);
-    d.counts = d.cell_start = d.tile_sums = nullptr;
+    if (d.counts) cudaFree(d.counts);  // the others lie in it
+    d.counts = d.cell_start = d.cell_head = d.tile_sums = nullptr;
     d.ncells = d.ncells_pad = d.ntiles = 0;
 }
 
@@ -206,17 +204,20 @@ sf_status alloc_grid(sf_ctx* ctx) {
     free_grid(d);
     const uint64_t pad = ((uint64_t)ctx->c.ncells + 1 + sf::kScanTile - 1) / sf::kScanTile * sf::kScanTile;
     const uint32_t ntiles = (uint32_t)(pad / sf::kScanTile);
-    cudaError_t e = dev_malloc(&d.counts, pad * sizeof(uint32_t));
-    if (e == cudaSuccess) e = dev_malloc(&d.cell_start, pad * sizeof(uint32_t));
-    if (e == cudaSuccess) e = dev_malloc(&d.tile_sums, (size_t)ntiles * sizeof(uint32_t));
-    if (e == cudaSuccess) e = cudaMemsetAsync(d.tile_sums, 0, (size_t)ntiles * sizeof(uint32_t), ctx->stream);
-    if (e == cudaSuccess) e = cudaMemsetAsync(d.counts, 0, pad * sizeof(uint32_t), ctx->stream);
-    if (e == cudaSuccess) e = cudaMemsetAsync(d.cell_start, 0, pad * sizeof(uint32_t), ctx->stream);
+    // one allocation: the histogram, the cell table, the scan-tile totals and,
+    // for small cells, the heads of their lists
+    const bool lists = ctx->c.reach >= sf::kListedReach;
+    const size_t words = 2 * pad + ntiles + (lists ? pad : 0);
+    cudaError_t e = dev_malloc(&d.counts, words * sizeof(uint32_t));
+    if (e == cudaSuccess) e = cudaMemsetAsync(d.counts, 0, (2 * pad + ntiles) * sizeof(uint32_t), ctx->stream);
     if (e != cudaSuccess) {
         free_grid(d);
         ctx->sorted = false;
         return cuda_fail(e, "grid allocation");
     }
+    d.cell_start = d.counts + pad;
+    d.tile_sums = d.cell_start + pad;
+    d.cell_head = lists ? d.tile_sums + ntiles : nullptr;
     d.ncells = ctx->c.ncells;
     d.ncells_pad = (uint32_t)pad;
     d.ntiles = ntiles;

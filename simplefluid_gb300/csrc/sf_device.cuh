@@ -212,12 +212,15 @@ __device__ __forceinline__ uint32_t checked_end(uint32_t v, uint32_t n) {
     uint64_t fn(bool) { return 0; }
 #endif
 
-// Counting-sort histogram: the particle's arrival slot in its cell, and the
-// cell's scan tile total (one atomic per distinct tile per warp).  Call with
-// every live lane of the warp converged.
-__device__ __forceinline__ uint32_t count_in_cell(uint32_t key, uint32_t* __restrict__ counts,
-                                                  uint32_t* __restrict__ tile_sums) {
-    const uint32_t slot = atomicAdd(counts + key, 1u);
+// Counting-sort histogram: particle i counted in its cell, and in the cell's
+// scan tile total (one atomic per distinct tile per warp).  Returns its arrival
+// slot in the cell or, with cell_head, the particle that was at the head of the
+// cell's list before it (undefined for the first).  Call with every live lane
+// of the warp converged.
+__device__ __forceinline__ uint32_t count_in_cell(uint32_t key, uint32_t i, uint32_t* __restrict__ counts,
+                                                  uint32_t* __restrict__ cell_head, uint32_t* __restrict__ tile_sums) {
+    const uint32_t slot = cell_head ? atomicExch(cell_head + key, i) : atomicAdd(counts + key, 1u);
+    if (cell_head) atomicAdd(counts + key, 1u);
     if (!tile_sums) return slot;  // the persistent batched step scans each scene without tile totals
     const unsigned mask = __activemask();
     const uint32_t tile = key / (uint32_t)kScanTile;

@@ -52,8 +52,8 @@ __global__ void __launch_bounds__(kBlockSize, (kPrefetch == 2 ? 1152 : 896) / kB
             const uint32_t* __restrict__ cs, const uint32_t* __restrict__ nbr, const uint32_t* __restrict__ nbr_count,
             const uint8_t* __restrict__ nbr_wide, const float4* __restrict__ pv, uint32_t n, SimConst c0, const SimConst* __restrict__ table, const uint32_t* __restrict__ scene_off,
             uint32_t nscenes, float4* __restrict__ pos_out, float4* __restrict__ vel_out,
-            uint32_t* __restrict__ counts, uint32_t* __restrict__ tile_sums, uint2* __restrict__ key_slot,
-            float4* __restrict__ acc_out, float4* __restrict__ sums, FrameState* __restrict__ frame) {
+            uint32_t* __restrict__ counts, uint32_t* __restrict__ cell_head, uint32_t* __restrict__ tile_sums,
+            uint2* __restrict__ key_slot, float4* __restrict__ acc_out, float4* __restrict__ sums, FrameState* __restrict__ frame) {
     grid_dependency_wait();
     allow_dependents();
     const uint32_t i = blockIdx.x * kBlockSize + threadIdx.x;
@@ -62,7 +62,7 @@ __global__ void __launch_bounds__(kBlockSize, (kPrefetch == 2 ? 1152 : 896) / kB
         force_one<kList, kPrefetch, kIntegrate, kReach, kBatched>(i, pos, vel, pr, cs, nbr, nbr_count, nbr_wide, pv, n, c0,
                                                                   table,
                                                                      scene_off, nscenes, pos_out, vel_out, counts,
-                                                                     tile_sums, key_slot, acc_out, sums, frame, v2, a2);
+                                                                     cell_head, tile_sums, key_slot, acc_out, sums, frame, v2, a2);
     if (!kBatched && kIntegrate && frame && c0.adaptive) raise_maxima<kBlockSize>(frame, v2, a2);
 }
 
@@ -72,8 +72,8 @@ __global__ void __launch_bounds__(kTeam * 32)
                  const uint32_t* __restrict__ cs, const uint32_t* __restrict__ nbr,
                  const uint32_t* __restrict__ nbr_count, const float4* __restrict__ pv, uint32_t n, SimConst c,
                  float4* __restrict__ pos_out, float4* __restrict__ vel_out, uint32_t* __restrict__ counts,
-                 uint32_t* __restrict__ tile_sums, uint2* __restrict__ key_slot, float4* __restrict__ acc_out,
-                 float4* __restrict__ sums, FrameState* __restrict__ frame) {
+                 uint32_t* __restrict__ cell_head, uint32_t* __restrict__ tile_sums, uint2* __restrict__ key_slot,
+                 float4* __restrict__ acc_out, float4* __restrict__ sums, FrameState* __restrict__ frame) {
     __shared__ ForceTeamShared sh;
     grid_dependency_wait();
     allow_dependents();
@@ -99,8 +99,8 @@ __global__ void __launch_bounds__(kTeam * 32)
             sums[2 * (size_t)i] = make_float4(a.apx, a.apy, a.apz, 0.f);
             sums[2 * (size_t)i + 1] = make_float4(a.avx, a.avy, a.avz, 0.f);
         }
-        force_finish<kIntegrate>(i, c, xi, vi, pri.y, a, pos_out, vel_out, counts, tile_sums, key_slot, acc_out, frame,
-                                 v2, a2);
+        force_finish<kIntegrate>(i, c, xi, vi, pri.y, a, pos_out, vel_out, counts, cell_head, tile_sums, key_slot,
+                                 acc_out, frame, v2, a2);
     }
     if (kIntegrate && frame && c.adaptive) raise_maxima<kTeam * 32>(frame, v2, a2);
 }
@@ -111,7 +111,7 @@ void force_team_as(DeviceState& d, const SimConst& c, cudaStream_t s) {
         launch_chained(k_force_team<kIntegrate, decltype(R)::value, kTeam, kTurn>, grid_for(d.n, kTeamParticles),
                        kTeam * 32, s, d.pos, d.vel, d.pr, d.cell_start, d.nbr, d.nbr_count, d.pv, d.n, c,
                        kIntegrate ? d.pos2 : nullptr, kIntegrate ? d.vel2 : nullptr, kIntegrate ? d.counts : nullptr,
-                       kIntegrate ? d.tile_sums : nullptr, kIntegrate ? d.key_slot : nullptr,
+                       kIntegrate ? d.cell_head : nullptr, kIntegrate ? d.tile_sums : nullptr, kIntegrate ? d.key_slot : nullptr,
                        kIntegrate ? nullptr : d.accel, d.sums, kIntegrate ? d.frame : nullptr);
     });
 }
@@ -127,6 +127,7 @@ void force_as(DeviceState& d, const SimConst& c, cudaStream_t s) {
         float4* po = kIntegrate ? d.pos2 : nullptr;
         float4* vo = kIntegrate ? d.vel2 : nullptr;
         uint32_t* co = kIntegrate ? d.counts : nullptr;
+        uint32_t* ch = kIntegrate ? d.cell_head : nullptr;
         uint32_t* ts = kIntegrate ? d.tile_sums : nullptr;
         uint2* ks = kIntegrate ? d.key_slot : nullptr;
         float4* ac = kIntegrate ? nullptr : d.accel;
@@ -135,12 +136,12 @@ void force_as(DeviceState& d, const SimConst& c, cudaStream_t s) {
                 launch_chained_window(win, k_force<kList, kPrefetch, kBlockSize, kIntegrate, K, true>,
                                grid_for(d.n, kBlockSize), kBlockSize, s, d.pos, d.vel, d.pr, d.cell_start, d.nbr,
                                d.nbr_count, d.nbr_wide, d.pv, d.n, c, d.table,
-                               d.scene_off, d.nscenes, po, vo, co, ts, ks, ac, d.sums, (FrameState*)nullptr);
+                               d.scene_off, d.nscenes, po, vo, co, ch, ts, ks, ac, d.sums, (FrameState*)nullptr);
         } else {
             launch_chained_window(win, k_force<kList, kPrefetch, kBlockSize, kIntegrate, K, false>,
                            grid_for(d.n, kBlockSize), kBlockSize, s, d.pos, d.vel, d.pr, d.cell_start, d.nbr,
                            d.nbr_count, d.nbr_wide, d.pv, d.n, c,
-                           (const SimConst*)nullptr, (const uint32_t*)nullptr, 0u, po, vo, co, ts, ks, ac, d.sums,
+                           (const SimConst*)nullptr, (const uint32_t*)nullptr, 0u, po, vo, co, ch, ts, ks, ac, d.sums,
                            kIntegrate ? d.frame : nullptr);
         }
     });

@@ -8,6 +8,8 @@
 // of the same scan that places the particles.  Stability (equal keys keep their
 // previous order) is restored by ranking each particle among its cell's
 // members, which makes the order deterministic and identical to a stable sort.
+// The members are found by the list that the histogram pass threads through
+// them or, in cells of the kernel radius's size, by bucketing their indices.
 #include <mutex>
 
 #include "sf_device.cuh"
@@ -137,8 +139,8 @@ template <bool kBatched>
 __global__ void k_load_hash(const float* __restrict__ pos3, const float* __restrict__ vel3, uint32_t n, SimConst c0,
                             const SimConst* __restrict__ table, const uint32_t* __restrict__ scene_off,
                             uint32_t nscenes, float4* __restrict__ pos, float4* __restrict__ vel,
-                            uint32_t* __restrict__ counts, uint32_t* __restrict__ tile_sums,
-                            uint2* __restrict__ key_slot) {
+                            uint32_t* __restrict__ counts, uint32_t* __restrict__ cell_head,
+                            uint32_t* __restrict__ tile_sums, uint2* __restrict__ key_slot) {
     allow_dependents();
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
@@ -152,21 +154,21 @@ __global__ void k_load_hash(const float* __restrict__ pos3, const float* __restr
         else
             vel[i] = make_float4(0.f, 0.f, 0.f, 0.f);
     }
-    key_slot[i] = make_uint2(key, count_in_cell(key, counts, tile_sums));
+    key_slot[i] = make_uint2(key, count_in_cell(key, i, counts, cell_head, tile_sums));
 }
 
 // Histogram of a loaded (not cell-sorted) state.
 template <bool kBatched>
 __global__ void k_hash_count(const float4* __restrict__ pos, uint32_t n, SimConst c0, const SimConst* __restrict__ table,
                              const uint32_t* __restrict__ scene_off, uint32_t nscenes, uint32_t* __restrict__ counts,
-                             uint2* __restrict__ key_slot) {
+                             uint32_t* __restrict__ cell_head, uint2* __restrict__ key_slot) {
     allow_dependents();
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     const SimConst c = const_of<kBatched>(c0, table, scene_off, nscenes, i);
     const float4 p = pos[i];
     const uint32_t key = cell_key(c, p.x, p.y, p.z);
-    key_slot[i] = make_uint2(key, atomicAdd(counts + key, 1u));
+    key_slot[i] = make_uint2(key, count_in_cell(key, i, counts, cell_head, nullptr));
 }
 
 template <bool kBatched>
@@ -190,85 +192,104 @@ __device__ __forceinline__ uint32_t warp_inclusive(uint32_t x) {
     return x;
 }
 
-// Exclusive scan over a 1024-thread block; *total receives the block sum.
-__device__ __forceinline__ uint32_t block_exclusive(uint32_t v, uint32_t* total) {
-    __shared__ uint32_t warp_sums[32];
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const uint32_t inc = warp_inclusive(v);
-    if (lane == 31) warp_sums[warp] = inc;
-    __syncthreads();
-    if (warp == 0) {
-        const uint32_t w = warp_sums[lane];
-        const uint32_t wi = warp_inclusive(w);
-        warp_sums[lane] = wi - w;
-        if (lane == 31) *total = wi;
-    }
-    __syncthreads();
-    const uint32_t r = warp_sums[warp] + inc - v;
-    __syncthreads();
-    return r;
-}
+__device__ __forceinline__ uint32_t sum4(const uint4& q) { return q.x + q.y + q.z + q.w; }
 
 // Tile totals of the cell histogram (one block per scan tile).
 __global__ void __launch_bounds__(kScanThreads) k_tile_totals(const uint4* __restrict__ counts,
                                                               uint32_t* __restrict__ tile_sums) {
-    __shared__ uint32_t total;
+    __shared__ uint32_t s_warp[kScanWarps];
     grid_dependency_wait();
     allow_dependents();
-    const uint4 q = counts[(size_t)blockIdx.x * kScanThreads + threadIdx.x];
-    block_exclusive(q.x + q.y + q.z + q.w, &total);
-    if (threadIdx.x == 0) tile_sums[blockIdx.x] = total;
+    uint32_t sum = 0;
+#pragma unroll
+    for (int k = 0; k < kScanChunks; ++k)
+        sum += sum4(counts[((size_t)blockIdx.x * kScanChunks + k) * kScanThreads + threadIdx.x]);
+    sum = __reduce_add_sync(0xffffffffu, sum);
+    if ((threadIdx.x & 31) == 0) s_warp[threadIdx.x >> 5] = sum;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        for (int w = 1; w < kScanWarps; ++w) sum += s_warp[w];
+        tile_sums[blockIdx.x] = sum;
+    }
 }
 
 // Exclusive scan of the cell histogram into the cell table, in one kernel.
-// Block b scans the contiguous scan tiles [t0, t1) (kScanTile cells each; a
-// few blocks per SM): it sums the totals of the tiles before t0 once (the
-// histogram atomics accumulated them in tile_sums), then carries the running
-// offset from tile to tile, loading the next tile's counts while it scans the
-// current one.  Two barriers per tile; the warp totals alternate between two
+// Block b scans the contiguous scan tiles [t0, t1) (kScanTile cells each): it
+// sums the totals of the tiles before t0 once (the histogram atomics
+// accumulated them in tile_sums), then carries the running offset from tile to
+// tile.  A warp takes a contiguous part of the tile in chunks of 128 cells,
+// four to a lane; all its loads are in flight at once and the chunks' scans
+// interleave.  One barrier per tile; the warp totals alternate between two
 // shared buffers so that a tile's writes never meet the previous tile's reads.
-__global__ void __launch_bounds__(kScanThreads, kScanBlocksPerSM) k_scan(const uint4* __restrict__ counts,
-                                                                         const uint32_t* __restrict__ tile_sums,
-                                                                         uint32_t ntiles, uint32_t n,
-                                                                         uint4* __restrict__ cell_start) {
-    static_assert(kScanThreads == 1024, "one warp-sum slot per warp");
+//
+// Bound by memory (64 MB at 8 million cells: 9 us) in large grids.  The blocks
+// are small because of the kernels around it: blocks of 1024 threads filled
+// their SMs, so the next kernels' blocks, launched meanwhile, crowded on the
+// others; a sub-step of 65,536 particles (1 million cells) took 43.5 us with
+// 1024 threads and one with 128 takes 38.1, of 236,987 93.1 and 91.4, of
+// 1,048,576 226.2 and 225.2.
+__global__ void __launch_bounds__(kScanThreads) k_scan(const uint4* __restrict__ counts,
+                                                       const uint32_t* __restrict__ tile_sums, uint32_t ntiles,
+                                                       uint32_t n, uint4* __restrict__ cell_start) {
     grid_dependency_wait();
     allow_dependents();
-    __shared__ uint32_t s_warp[2][32], s_before[32];
+    __shared__ uint32_t s_warp[2][kScanWarps], s_before[kScanWarps];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const uint32_t per = (ntiles + gridDim.x - 1) / gridDim.x;
     const uint32_t t0 = blockIdx.x * per, t1 = min(t0 + per, ntiles);
     if (t0 >= t1) return;  // the whole block
-    uint4 q = counts[(size_t)t0 * kScanThreads + threadIdx.x];
+    constexpr size_t kTile4 = kScanTile / 4;
+    const size_t at = (size_t)t0 * kTile4 + warp * (kScanChunks * 32) + lane;
+    counts += at;
+    cell_start += at;
+    uint4 q[kScanChunks];
+#pragma unroll
+    for (int k = 0; k < kScanChunks; ++k) q[k] = counts[32 * k];
     uint32_t before = 0;
-    for (uint32_t k = threadIdx.x; k < t0; k += kScanThreads) before += tile_sums[k];
+    for (uint32_t k = threadIdx.x; k < t0 / 4; k += kScanThreads)
+        before += sum4(reinterpret_cast<const uint4*>(tile_sums)[k]);
+    if (threadIdx.x < t0 % 4) before += tile_sums[t0 - 1 - threadIdx.x];
     before = __reduce_add_sync(0xffffffffu, before);
     if (lane == 0) s_before[warp] = before;
     __syncthreads();
-    // warp 0 carries the offset of the current tile (the same in every lane)
-    uint32_t base = warp == 0 ? __reduce_add_sync(0xffffffffu, s_before[lane]) : 0u;
-    for (uint32_t t = t0; t < t1; ++t) {
+    uint32_t base = 0;  // particles in the cells of the earlier tiles
+#pragma unroll
+    for (int w = 0; w < kScanWarps; ++w) base += s_before[w];
+    for (uint32_t t = t0; t < t1; ++t, counts += kTile4, cell_start += kTile4) {
         uint32_t* const ws = s_warp[(t - t0) & 1];
-        uint4 qn = make_uint4(0u, 0u, 0u, 0u);
-        if (t + 1 < t1) qn = counts[(size_t)(t + 1) * kScanThreads + threadIdx.x];
-        const uint32_t v = q.x + q.y + q.z + q.w;
-        const uint32_t inc = warp_inclusive(v);
-        if (lane == 31) ws[warp] = inc;
-        __syncthreads();
-        if (warp == 0) {
-            const uint32_t w = ws[lane];
-            const uint32_t wi = warp_inclusive(w);
-            ws[lane] = wi - w + base;  // cells of the earlier warps and tiles
-            base += __shfl_sync(0xffffffffu, wi, 31);
+        if (t != t0) {
+#pragma unroll
+            for (int k = 0; k < kScanChunks; ++k) q[k] = counts[32 * k];
         }
+        uint32_t v[kScanChunks], inc[kScanChunks], sum = 0;
+#pragma unroll
+        for (int k = 0; k < kScanChunks; ++k) {
+            v[k] = sum4(q[k]);
+            inc[k] = warp_inclusive(v[k]);
+        }
+#pragma unroll
+        for (int k = 0; k < kScanChunks; ++k) {
+            v[k] = sum + inc[k] - v[k];  // exclusive within the warp's part
+            sum += __shfl_sync(0xffffffffu, inc[k], 31);
+        }
+        if (lane == 0) ws[warp] = sum;
         __syncthreads();
+        uint32_t first = base;
+#pragma unroll
+        for (int w = 0; w < kScanWarps; ++w) {
+            const uint32_t x = ws[w];
+            first += w < warp ? x : 0u;
+            base += x;
+        }
         // Entries are clamped to n: a histogram that does not sum to n (never
         // the case when each step's counts start from zero) cannot send the
         // candidate walks past the particle arrays.
-        const uint32_t ex = ws[warp] + inc - v;
-        cell_start[(size_t)t * kScanThreads + threadIdx.x] =
-            make_uint4(min(ex, n), min(ex + q.x, n), min(ex + q.x + q.y, n), min(ex + q.x + q.y + q.z, n));
-        q = qn;
+#pragma unroll
+        for (int k = 0; k < kScanChunks; ++k) {
+            const uint32_t ex = first + v[k];
+            cell_start[32 * k] = make_uint4(min(ex, n), min(ex + q[k].x, n), min(ex + q[k].x + q[k].y, n),
+                                            min(ex + q[k].x + q[k].y + q[k].z, n));
+        }
     }
 }
 
@@ -302,6 +323,38 @@ __global__ void k_rank_gather(const uint2* __restrict__ key_slot, const uint32_t
     const uint32_t b = cell_start[key], e = cell_start[key + 1];
     uint32_t rank = 0;
     for (uint32_t t = b; t < e; ++t) rank += (tmp[t] < i) ? 1u : 0u;
+    const uint32_t dst = b + rank;
+    if (dst < n) {  // always, unless the histogram was inconsistent
+        pos_out[dst] = p;
+        vel_out[dst] = v;
+    }
+}
+
+// Both in one where the cells have lists: a particle's rank is the number of
+// its list's entries below it.  The list needs no clearing (its length is in
+// the cell table) and up to two entries no walk: the head and the particle's
+// own link are read with the cell's range.
+__global__ void k_list_gather(const uint2* __restrict__ key_next, const uint32_t* __restrict__ cell_start,
+                              const uint32_t* __restrict__ cell_head, const float4* __restrict__ pos_in,
+                              const float4* __restrict__ vel_in, uint32_t n, float4* __restrict__ pos_out,
+                              float4* __restrict__ vel_out, uint32_t* __restrict__ counts,
+                              uint32_t* __restrict__ tile_sums, uint32_t ntiles) {
+    grid_dependency_wait();
+    allow_dependents();
+    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+    for (uint32_t t = i; t < ntiles; t += gridDim.x * blockDim.x) tile_sums[t] = 0u;
+    if (i >= n) return;
+    const float4 p = pos_in[i], v = vel_in[i];  // in flight while the rank is found
+    const uint2 kn = key_next[i];
+    const uint32_t b = cell_start[kn.x], e = cell_start[kn.x + 1];
+    uint32_t t = cell_head[kn.x], left = e - b, rank = 0;
+    counts[kn.x] = 0u;
+    // `left` entries not visited; the last need not be if it is the own one
+    for (uint32_t last = 1u; left > last && t < n; t = t == i ? kn.y : key_next[t].y) {
+        rank += t < i ? 1u : 0u;
+        if (t == i) last = 0u;
+        if (--left <= last) break;
+    }
     const uint32_t dst = b + rank;
     if (dst < n) {  // always, unless the histogram was inconsistent
         pos_out[dst] = p;
@@ -466,10 +519,10 @@ void launch_load_hash(const DeviceState& d, const float* pos3, const float* vel3
     uint32_t* const tiles = n < kTileAtomics ? d.tile_sums : nullptr;
     if (d.table)
         k_load_hash<true><<<grid_for(n, kBlock), kBlock, 0, s>>>(pos3, vel3, n, c, d.table, d.scene_off, d.nscenes,
-                                                                 d.pos2, vel, d.counts, tiles, d.key_slot);
+                                                                 d.pos2, vel, d.counts, d.cell_head, tiles, d.key_slot);
     else
         k_load_hash<false><<<grid_for(n, kBlock), kBlock, 0, s>>>(pos3, vel3, n, c, nullptr, nullptr, 0, d.pos2, vel,
-                                                                  d.counts, tiles, d.key_slot);
+                                                                  d.counts, d.cell_head, tiles, d.key_slot);
     if (!tiles) launch_tile_totals(d, d.counts, s);
 }
 
@@ -503,9 +556,10 @@ void launch_hash_count(const DeviceState& d, const float4* pos, uint32_t n, cons
     if (!n) return;
     if (d.table)
         k_hash_count<true><<<grid_for(n, kBlock), kBlock, 0, s>>>(pos, n, c, d.table, d.scene_off, d.nscenes, counts,
-                                                                  key_slot);
+                                                                  d.cell_head, key_slot);
     else
-        k_hash_count<false><<<grid_for(n, kBlock), kBlock, 0, s>>>(pos, n, c, nullptr, nullptr, 0, counts, key_slot);
+        k_hash_count<false><<<grid_for(n, kBlock), kBlock, 0, s>>>(pos, n, c, nullptr, nullptr, 0, counts, d.cell_head,
+                                                           key_slot);
     launch_tile_totals(d, counts, s);
 }
 
@@ -525,19 +579,20 @@ void launch_scan_cells(DeviceState& d, uint32_t /*n*/, cudaStream_t s) {
 }
 
 // Buckets indices by cell and clears the counters.
-void launch_scatter(const uint2* key_slot, const uint32_t* cell_start, uint32_t n, uint32_t* tmp, uint32_t* counts,
-                    cudaStream_t s) {
-    if (n) launch_chained(k_scatter, grid_for(n, kBlock), kBlock, s, key_slot, cell_start, n, tmp, counts);
+void launch_scatter(const DeviceState& d, cudaStream_t s) {
+    if (d.n && !d.cell_head)
+        launch_chained(k_scatter, grid_for(d.n, kBlock), kBlock, s, d.key_slot, d.cell_start, d.n, d.tmp, d.counts);
 }
 
-// Stable rank inside each cell and the gather; also zeroes the scan-tile
-// totals (ntiles entries) for the next histogram.
-void launch_rank_gather(const uint2* key_slot, const uint32_t* cell_start, const uint32_t* tmp, const float4* pos_in,
-                        const float4* vel_in, uint32_t n, float4* pos_out, float4* vel_out, uint32_t* tile_sums,
-                        uint32_t ntiles, cudaStream_t s) {
-    if (n)
-        launch_chained(k_rank_gather, grid_for(n, kBlock), kBlock, s, key_slot, cell_start, tmp, pos_in, vel_in, n,
-                       pos_out, vel_out, tile_sums, ntiles);
+// Stable rank inside each cell and the gather.
+void launch_rank_gather(const DeviceState& d, cudaStream_t s) {
+    if (!d.n) return;
+    if (d.cell_head)
+        launch_chained(k_list_gather, grid_for(d.n, kBlock), kBlock, s, d.key_slot, d.cell_start, d.cell_head, d.pos2,
+                       d.vel2, d.n, d.pos, d.vel, d.counts, d.tile_sums, d.ntiles);
+    else
+        launch_chained(k_rank_gather, grid_for(d.n, kBlock), kBlock, s, d.key_slot, d.cell_start, d.tmp, d.pos2,
+                       d.vel2, d.n, d.pos, d.vel, d.tile_sums, d.ntiles);
 }
 
 void launch_neighbour_stats(const DeviceState& d, const SimConst& c, uint32_t* count, uint32_t* hash,
@@ -558,9 +613,9 @@ void launch_neighbour_stats(const DeviceState& d, const SimConst& c, uint32_t* c
 
 void enqueue_sort_tail(DeviceState& d, cudaStream_t s, cudaEvent_t before_gather) {
     launch_scan_cells(d, d.n, s);
-    launch_scatter(d.key_slot, d.cell_start, d.n, d.tmp, d.counts, s);
+    launch_scatter(d, s);
     if (before_gather) cudaStreamWaitEvent(s, before_gather, 0);
-    launch_rank_gather(d.key_slot, d.cell_start, d.tmp, d.pos2, d.vel2, d.n, d.pos, d.vel, d.tile_sums, d.ntiles, s);
+    launch_rank_gather(d, s);
 }
 
 const char* const kStageNames[kNumStages] = {"density", "force_integrate", "scan", "scatter", "rank_gather"};
@@ -570,11 +625,8 @@ void enqueue_stage(uint32_t stage, DeviceState& d, const SimConst& c, cudaStream
         case 0: launch_density(d, c, s); break;
         case 1: launch_force_integrate(d, c, s); break;
         case 2: launch_scan_cells(d, d.n, s); break;
-        case 3: launch_scatter(d.key_slot, d.cell_start, d.n, d.tmp, d.counts, s); break;
-        case 4:
-            launch_rank_gather(d.key_slot, d.cell_start, d.tmp, d.pos2, d.vel2, d.n, d.pos, d.vel, d.tile_sums,
-                               d.ntiles, s);
-            break;
+        case 3: launch_scatter(d, s); break;
+        case 4: launch_rank_gather(d, s); break;
         default: break;
     }
 }

@@ -96,8 +96,8 @@ struct DeviceState {
     float4* vel2 = nullptr;
     float2* pr = nullptr;    // (pressure, 1/density) of the last density pass
     float* rho = nullptr;    // density of the last density pass
-    uint2* key_slot = nullptr;  // (cell key, arrival slot) of pos2/vel2 order
-    uint32_t* tmp = nullptr;    // cell-bucketed unsorted indices
+    uint2* key_slot = nullptr;  // (cell key, arrival slot or next of the cell's list) of pos2/vel2 order
+    uint32_t* tmp = nullptr;    // scratch; without cell_head, the cell-bucketed unsorted indices
     float* io = nullptr;        // AoS staging, 6 floats per particle
     float4* accel = nullptr;    // optional acceleration output (inspection)
     uint32_t* nbr = nullptr;       // neighbour lists, tile-major (kNbCap * kNbTile per tile)
@@ -109,8 +109,12 @@ struct DeviceState {
     // grid
     uint32_t ncells = 0, ncells_pad = 0;
     uint32_t* counts = nullptr;      // ncells_pad, zero between steps
-    // per scan tile (kScanTile cells): particles counted in it, zero between steps
     uint32_t* cell_start = nullptr;  // ncells + 1
+    // ncells_pad, or null: the heads of the lists that the particles of a cell
+    // form in arrival order (key_slot holds the links), defined where counts
+    // is not zero
+    uint32_t* cell_head = nullptr;
+    // per scan tile (kScanTile cells): particles counted in it, zero between steps
     uint32_t* tile_sums = nullptr;
     uint32_t ntiles = 0;
     // batches of independent scenes (null for a single scene): per-scene
@@ -124,16 +128,17 @@ struct DeviceState {
     uint32_t* scene_queue = nullptr;
 };
 
-constexpr int kScanThreads = 1024;
-constexpr int kScanItems = 4;
-constexpr int kScanTile = kScanThreads * kScanItems;
+constexpr int kScanTile = 4096;
+constexpr int kScanThreads = 128;
+constexpr int kScanWarps = kScanThreads / 32;
+constexpr int kScanChunks = kScanTile / 4 / kScanThreads;  // groups of four cells per thread
 // Uploads of fewer particles count their scan tiles with one atomic per tile
 // and warp; larger ones sum the histogram in a launch of its own
 // (k_tile_totals).  Upload and sort, atomics / own launch: 16,000 particles
 // 13.3 / 15.3 us, 65,536 13.6 / 15.2 in rows but 24.6 / 16.9 in random order,
 // where a warp's lanes hit 32 tiles and the atomics contend (236,987: 67 / 29).
 constexpr uint32_t kTileAtomics = 32768;
-constexpr int kScanBlocksPerSM = 2;  // resident scan blocks per SM (the scan grid's size)
+constexpr int kScanBlocksPerSM = 8;  // the scan grid's size
 
 // Persisting L2 (sf_grid.cu).  reserve_persisting_l2(want) grows this
 // process's persisting-L2 carve-out on the current device to `want` bytes
@@ -164,12 +169,16 @@ void launch_store_caller_order(const float4* pos, const float4* vel, uint32_t n,
 void launch_hash_count(const DeviceState& d, const float4* pos, uint32_t n, const SimConst& c, uint32_t* counts,
                        uint2* key_slot, cudaStream_t s);
 void launch_scan_cells(DeviceState& d, uint32_t n, cudaStream_t s);
-void launch_scatter(const uint2* key_slot, const uint32_t* cell_start, uint32_t n, uint32_t* tmp, uint32_t* counts,
-                    cudaStream_t s);
-// also zeroes tile_sums (ntiles entries) for the next histogram
-void launch_rank_gather(const uint2* key_slot, const uint32_t* cell_start, const uint32_t* tmp, const float4* pos_in,
-                        const float4* vel_in, uint32_t n, float4* pos_out, float4* vel_out, uint32_t* tile_sums,
-                        uint32_t ntiles, cudaStream_t s);
+// nothing where cells have lists (cell_head)
+void launch_scatter(const DeviceState& d, cudaStream_t s);
+// also zeroes tile_sums for the next histogram
+void launch_rank_gather(const DeviceState& d, cudaStream_t s);
+// Cells of this many per kernel radius or more (at rest one particle a cell)
+// are sorted through lists, one launch less: a sub-step of 16,000 particles
+// 18.2 -> 16.7 us, of 236,987 95 -> 93, of 1,048,576 227.8 -> 226.3.  A cell of
+// the kernel radius itself holds eight, and its list would be walked entry by
+// entry; there the indices are bucketed (k_scatter) and read side by side.
+constexpr int kListedReach = 2;
 // Scenes of fewer particles take the team forms (sf_team.cuh) of the two
 // passes.  Stage times in us, one thread per particle against the team
 // (jittered lattice; disordered): density 16.4 / 10.3 at 16,000 particles,

@@ -9,7 +9,7 @@
 // caller hands in its own position and output buffers; everything else this
 // computation needs lives in g_sf_noalloc_scratch below.
 //
-// Scratch: one static __device__ array of kNoAllocScratchBytes (about 7.6 MB).
+// Scratch: one static __device__ array of kNoAllocScratchBytes (about 8.3 MB).
 // Every GPU that loads this library holds it until the process exits.  It caps
 // a call at kNoAllocMaxParticles particles and kNoAllocMaxCells grid cells;
 // larger requests are rejected with SF_ERR_CAPACITY before any GPU work.
@@ -54,7 +54,8 @@ constexpr uint64_t kOffPr = kOffVel2 + align256(16ull * kNoAllocMaxParticles);
 constexpr uint64_t kOffRho = kOffPr + align256(8ull * kNoAllocMaxParticles);
 constexpr uint64_t kOffKeySlot = kOffRho + align256(4ull * kNoAllocMaxParticles);
 constexpr uint64_t kOffTmp = kOffKeySlot + align256(8ull * kNoAllocMaxParticles);
-constexpr uint64_t kOffCounts = kOffTmp + align256(4ull * kNoAllocMaxParticles);
+constexpr uint64_t kOffCounts =
+    kOffTmp + align256(4ull * (kNoAllocCellsPad > kNoAllocMaxParticles ? kNoAllocCellsPad : kNoAllocMaxParticles));
 constexpr uint64_t kOffCellStart = kOffCounts + align256(4ull * kNoAllocCellsPad);
 constexpr uint64_t kOffTileSums = kOffCellStart + align256(4ull * kNoAllocCellsPad);
 constexpr uint64_t kNoAllocScratchBytes = kOffTileSums + align256(4ull * kNoAllocTiles);
@@ -156,7 +157,8 @@ int noalloc_density(const sf_params& p, const SimConst& c, const float* d_pos_xy
     d.pr = reinterpret_cast<float2*>(base + kOffPr);
     d.rho = reinterpret_cast<float*>(base + kOffRho);
     d.key_slot = reinterpret_cast<uint2*>(base + kOffKeySlot);
-    d.tmp = reinterpret_cast<uint32_t*>(base + kOffTmp);
+    // the cells' lists, or the bucketed indices
+    (c.reach >= kListedReach ? d.cell_head : d.tmp) = reinterpret_cast<uint32_t*>(base + kOffTmp);
     d.counts = reinterpret_cast<uint32_t*>(base + kOffCounts);
     d.cell_start = reinterpret_cast<uint32_t*>(base + kOffCellStart);
     d.tile_sums = reinterpret_cast<uint32_t*>(base + kOffTileSums);

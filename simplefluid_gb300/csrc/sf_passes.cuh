@@ -194,7 +194,8 @@ template <bool kIntegrate>
 __device__ __forceinline__ void force_finish(uint32_t i, const SimConst& c, const float4& xi, const float4& vi,
                                              float inv, const PairAcc& a, float4* __restrict__ pos_out,
                                              float4* __restrict__ vel_out, uint32_t* __restrict__ counts,
-                                             uint32_t* __restrict__ tile_sums, uint2* __restrict__ key_slot,
+                                             uint32_t* __restrict__ cell_head, uint32_t* __restrict__ tile_sums,
+                                             uint2* __restrict__ key_slot,
                                              float4* __restrict__ acc_out, const FrameState* __restrict__ frame,
                                              uint32_t& v2, uint32_t& a2) {
     const float ax = fmaf(fmaf(c.cp, a.apx, c.cv * a.avx), inv, c.g[0]);
@@ -221,7 +222,7 @@ __device__ __forceinline__ void force_finish(uint32_t i, const SimConst& c, cons
     pos_out[i] = make_float4(x[0], x[1], x[2], xi.w);
     vel_out[i] = make_float4(v[0], v[1], v[2], 0.f);
     const uint32_t key = cell_key(c, x[0], x[1], x[2]);
-    key_slot[i] = make_uint2(key, count_in_cell(key, counts, tile_sums));
+    key_slot[i] = make_uint2(key, count_in_cell(key, i, counts, cell_head, tile_sums));
     if (frame && c.adaptive) {
         v2 = max(v2, __float_as_uint(fmaf(v[2], v[2], fmaf(v[1], v[1], v[0] * v[0]))));
         a2 = max(a2, __float_as_uint(fmaf(az, az, fmaf(ay, ay, ax * ax))));
@@ -232,8 +233,8 @@ __device__ __forceinline__ void force_finish(uint32_t i, const SimConst& c, cons
 // histogram entry, or (!kIntegrate) its acceleration.  With the adaptive
 // sub-step, v2 and a2 are raised to |v'|^2 and |a|^2 (float bits).
 // kList: 0 no list (rescan), 1 32-bit entries, 2 16-bit entries (32-bit in
-// warp tiles marked in nbr_wide).  tile_sums may be null (no scan-tile
-// totals).
+// warp tiles marked in nbr_wide).  cell_head and tile_sums may be null (arrival
+// slots instead of cell lists; no scan-tile totals).
 template <int kList, int kPrefetch, bool kIntegrate, int kReach, bool kBatched, bool kNc = true>
 __device__ __forceinline__ void force_one(
     uint32_t i, const float4* __restrict__ pos, const float4* __restrict__ vel, const float2* __restrict__ pr,
@@ -241,7 +242,8 @@ __device__ __forceinline__ void force_one(
     const uint8_t* __restrict__ nbr_wide, const float4* __restrict__ pv, uint32_t n, const SimConst& c0,
     const SimConst* __restrict__ table, const uint32_t* __restrict__ scene_off, uint32_t nscenes,
     float4* __restrict__ pos_out, float4* __restrict__ vel_out, uint32_t* __restrict__ counts,
-    uint32_t* __restrict__ tile_sums, uint2* __restrict__ key_slot, float4* __restrict__ acc_out,
+    uint32_t* __restrict__ cell_head, uint32_t* __restrict__ tile_sums, uint2* __restrict__ key_slot,
+    float4* __restrict__ acc_out,
     float4* __restrict__ sums, const FrameState* __restrict__ frame, uint32_t& v2, uint32_t& a2) {
     // A batch reads its scene's constants where they are used (the kernel
     // radius before the neighbour loop, the rest after it) instead of
@@ -295,7 +297,7 @@ __device__ __forceinline__ void force_one(
         sums[2 * (size_t)i] = make_float4(a.apx, a.apy, a.apz, 0.f);
         sums[2 * (size_t)i + 1] = make_float4(a.avx, a.avy, a.avz, 0.f);
     }
-    force_finish<kIntegrate>(i, c, xi, vi, pri.y, a, pos_out, vel_out, counts, tile_sums, key_slot, acc_out, frame, v2,
+    force_finish<kIntegrate>(i, c, xi, vi, pri.y, a, pos_out, vel_out, counts, cell_head, tile_sums, key_slot, acc_out, frame, v2,
                              a2);
 }
 

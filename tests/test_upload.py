@@ -34,3 +34,27 @@ def test_state_comes_back_as_uploaded(n, where):
                 assert np.array_equal(a.view(np.uint32), b.view(np.uint32))
             report = s.checkState()
             assert not report["unsorted"] and not report["cell_table_mismatch"] and not report["bad_ids"], report
+
+
+@pytest.mark.parametrize("cells", [1, 2, 3])
+@pytest.mark.parametrize("per_cell", [1, 2, 3, 7, 300])
+def test_cells_of_any_size_sort_stably(cells, per_cell):
+    rng = np.random.default_rng(per_cell)
+    n = 3000
+    spots = rng.random((n // per_cell, 3)).astype(np.float32)
+    pos = spots[rng.permutation(np.arange(n) % len(spots))]  # coincident particles, no order at all
+    vel = rng.normal(size=(n, 3)).astype(np.float32)
+    prm = params_16k(cellsPerH=cells)
+    with SPHSolver(prm) as s:
+        for _ in range(2):
+            s.setParticles(pos, vel)
+            spos, svel, ids, keys = s.sortedState()
+            of = np.empty(n, np.uint32)
+            of[ids] = keys
+            assert np.array_equal(ids, np.argsort(of, kind="stable"))
+            assert np.array_equal(spos, pos[ids]) and np.array_equal(svel, vel[ids])
+            counts = np.bincount(keys, minlength=s.cellStart().size - 1)
+            assert np.array_equal(s.cellStart(), np.concatenate([[0], np.cumsum(counts)]).astype(np.uint32))
+            s.step(1)  # the next histogram is the force pass's
+            spos, svel, ids, keys = s.sortedState()
+            assert (np.diff(keys.astype(np.int64)) >= 0).all() and s.checkState()["cell_table_mismatch"] == 0
