@@ -41,7 +41,7 @@ __global__ void __launch_bounds__(kBlockSize)
               float4* __restrict__ pv, FrameState* __restrict__ frame) {
     __shared__ uint32_t s_nb[kMode == kEmitStaged ? kNbCap : 1][kMode == kEmitStaged ? kBlockSize : 1];
     grid_dependency_wait();
-    allow_dependents();
+    allow_dependents_sized(n);
     // a stepping pass with a frame state chooses this sub-step's dt
     if (frame && blockIdx.x == 0 && threadIdx.x == 0) choose_dt(frame, c0);
     const uint32_t t = threadIdx.x;
@@ -76,7 +76,7 @@ __global__ void __launch_bounds__((2 * kReach + 1) * 32)
                    FrameState* __restrict__ frame) {
     __shared__ DensityTeamShared<kReach> sh;
     grid_dependency_wait();
-    allow_dependents();
+    allow_dependents_sized(n);
     if (frame && blockIdx.x == 0 && threadIdx.x == 0) choose_dt(frame, c);
     const uint32_t i = blockIdx.x * kTeamParticles + (threadIdx.x & 31u);
     density_team<kReach>(min(i, n - 1), i < n, c, pos, cs, n, rho_out, pr_out, nbr, nbr_count, vel, pv, sh);

@@ -55,7 +55,7 @@ __global__ void __launch_bounds__(kBlockSize, (kPrefetch == 2 ? 1152 : 896) / kB
             uint32_t* __restrict__ counts, uint32_t* __restrict__ cell_head, uint32_t* __restrict__ tile_sums,
             uint2* __restrict__ key_slot, float4* __restrict__ acc_out, float4* __restrict__ sums, FrameState* __restrict__ frame) {
     grid_dependency_wait();
-    allow_dependents();
+    allow_dependents_sized(n);
     const uint32_t i = blockIdx.x * kBlockSize + threadIdx.x;
     uint32_t v2 = 0u, a2 = 0u;
     if (i < n)

@@ -340,7 +340,6 @@ __global__ void k_list_gather(const uint2* __restrict__ key_next, const uint32_t
                               float4* __restrict__ vel_out, uint32_t* __restrict__ counts,
                               uint32_t* __restrict__ tile_sums, uint32_t ntiles) {
     grid_dependency_wait();
-    allow_dependents();
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     for (uint32_t t = i; t < ntiles; t += gridDim.x * blockDim.x) tile_sums[t] = 0u;
     if (i >= n) return;
@@ -355,6 +354,9 @@ __global__ void k_list_gather(const uint2* __restrict__ key_next, const uint32_t
         if (t == i) last = 0u;
         if (--left <= last) break;
     }
+    // not before: the density pass's blocks would crowd on the SMs that this
+    // kernel leaves free (20 sub-steps of 16,000 particles 333 -> 304 us)
+    allow_dependents();
     const uint32_t dst = b + rank;
     if (dst < n) {  // always, unless the histogram was inconsistent
         pos_out[dst] = p;

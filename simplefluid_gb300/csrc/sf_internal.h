@@ -186,6 +186,8 @@ constexpr int kListedReach = 2;
 // force 12.3 / 9.5 at 16,000, 12.9 / 12.3; 14.7 / 14.3 at 32,000, 13.1 / 16.1
 // at 48,000.
 constexpr uint32_t kDensityTeamScene = 57344, kForceTeamScene = 32768;
+// Scenes from this size on launch the next pass early (allow_dependents_sized).
+constexpr uint32_t kEarlyLaunchScene = 196608;
 // Warps per 32 particles in the force pass, and neighbours they take in turn
 // (2 x 4; stage times at 16,000 and 32,000 particles 9.5 and 12.3 us, 4 x 4
 // 9.6 and 13.7, 3 x 2 9.6 and 13.9, 8 x 2 12.4 and 15.6).
