@@ -939,8 +939,31 @@ SF_API sf_status sf_advance_frame(sf_ctx* ctx, float* dt_out) {
     return SF_OK;
 }
 
-// One frame as a graph: reset the frame clock, then a conditional while node
-// whose body is one sub-step followed by the frame check.
+// A conditional while node behind `after` (whose place it takes), its body
+// `own.run` sub-steps and the frame check.
+static sf_status add_frame_loop(sf_ctx* ctx, cudaGraph_t g, std::vector<cudaGraphNode_t>& after,
+                                const sf::FrameLimits& limits, const sf::FrameLoop& own, const sf::FrameLoop& next) {
+    cudaGraphNodeParams cp = {};
+    cp.type = cudaGraphNodeTypeConditional;
+    cp.conditional.handle = own.h;
+    cp.conditional.type = cudaGraphCondTypeWhile;
+    cp.conditional.size = 1;
+    cudaGraphNode_t cn;
+    SF_CUDA(cudaGraphAddNode(&cn, g, after.data(), nullptr, after.size(), &cp));
+    after.assign(1, cn);
+    cudaGraph_t body = cp.conditional.phGraph_out[0];
+    SF_CUDA(cudaStreamBeginCaptureToGraph(ctx->stream, body, nullptr, nullptr, 0, cudaStreamCaptureModeThreadLocal));
+    sf::DeviceState dr = ctx->d;
+    dr.frame = ctx->frame;  // the density pass chooses dt, the force pass reads it
+    for (uint32_t k = 0; k < own.run; ++k) sf::enqueue_step(dr, ctx->c, ctx->stream);
+    sf::launch_frame_check(ctx->frame, limits, own, next, ctx->stream);
+    SF_CUDA(cudaStreamEndCapture(ctx->stream, &body));
+    return SF_OK;
+}
+
+// One frame as a graph: reset the frame clock, then conditional while nodes:
+// runs of sub-steps (of the lengths a frame has room for), then single ones up
+// to the frame's end.
 static sf_status build_frame_graph(sf_ctx* ctx, double frame_time, uint32_t max_substeps, cudaGraphExec_t* out) {
     cudaGraph_t g = nullptr;
     SF_CUDA(cudaGraphCreate(&g, 0));
@@ -950,30 +973,27 @@ static sf_status build_frame_graph(sf_ctx* ctx, double frame_time, uint32_t max_
             if (g) cudaGraphDestroy(g);
         }
     } guard{g};
-    cudaGraphConditionalHandle h;
-    SF_CUDA(cudaGraphConditionalHandleCreate(&h, g, 1, cudaGraphCondAssignDefault));
+    const sf::FrameLimits limits{frame_time, ctx->c.dt, max_substeps};
+    sf::FrameLoop runs[2], single;
+    uint32_t nruns = 0;
+    for (const uint32_t run : sf::kFrameRuns) {
+        if (!(run * (double)ctx->c.dt < frame_time && run < max_substeps)) continue;
+        runs[nruns].run = run;
+        SF_CUDA(cudaGraphConditionalHandleCreate(&runs[nruns++].h, g, 0, cudaGraphCondAssignDefault));
+    }
+    single.run = 1;
+    SF_CUDA(cudaGraphConditionalHandleCreate(&single.h, g, 1, cudaGraphCondAssignDefault));
     SF_CUDA(cudaStreamBeginCaptureToGraph(ctx->stream, g, nullptr, nullptr, 0, cudaStreamCaptureModeThreadLocal));
-    sf::launch_frame_begin(ctx->frame, ctx->stream);
+    sf::launch_frame_begin(ctx->frame, limits, runs[0], runs[1], ctx->stream);
     cudaGraph_t captured = nullptr;
     SF_CUDA(cudaStreamEndCapture(ctx->stream, &captured));
     size_t nn = 0;
     SF_CUDA(cudaGraphGetNodes(g, nullptr, &nn));
     std::vector<cudaGraphNode_t> nodes(nn);
     SF_CUDA(cudaGraphGetNodes(g, nodes.data(), &nn));
-    cudaGraphNodeParams cp = {};
-    cp.type = cudaGraphNodeTypeConditional;
-    cp.conditional.handle = h;
-    cp.conditional.type = cudaGraphCondTypeWhile;
-    cp.conditional.size = 1;
-    cudaGraphNode_t cn;
-    SF_CUDA(cudaGraphAddNode(&cn, g, nodes.data(), nullptr, nn, &cp));
-    cudaGraph_t body = cp.conditional.phGraph_out[0];
-    SF_CUDA(cudaStreamBeginCaptureToGraph(ctx->stream, body, nullptr, nullptr, 0, cudaStreamCaptureModeThreadLocal));
-    sf::DeviceState dr = ctx->d;
-    dr.frame = ctx->frame;  // the density pass chooses dt, the force pass reads it
-    sf::enqueue_step(dr, ctx->c, ctx->stream);
-    sf::launch_frame_check(ctx->frame, frame_time, max_substeps, h, ctx->stream);
-    SF_CUDA(cudaStreamEndCapture(ctx->stream, &body));
+    for (uint32_t k = 0; k < nruns; ++k)
+        SF_TRY(add_frame_loop(ctx, g, nodes, limits, runs[k], k + 1 < nruns ? runs[k + 1] : sf::FrameLoop{}));
+    SF_TRY(add_frame_loop(ctx, g, nodes, limits, single, sf::FrameLoop{}));
     SF_CUDA(cudaGraphInstantiate(out, g, 0));
     return SF_OK;
 }

@@ -419,7 +419,8 @@ __device__ __forceinline__ void st8(float4* __restrict__ p, const float4& a, con
 }
 
 // The sub-step's dt from the previous sub-step's maxima (adaptive: CFL on
-// |v| and |a|; fixed: time_step), then the maxima restart for this sub-step.
+// |v| and |a|; fixed: time_step), counted into the frame clock; then the maxima
+// restart for this sub-step.
 __device__ __forceinline__ void choose_dt(FrameState* __restrict__ fs, const SimConst& c) {
     float dt = c.dt;
     if (c.adaptive) {
@@ -428,6 +429,9 @@ __device__ __forceinline__ void choose_dt(FrameState* __restrict__ fs, const Sim
         if (a2 > 0.f) dt = fminf(dt, c.cfl_a * sqrtf(c.h / sqrtf(a2)));
     }
     fs->dt = dt;
+    fs->frame_acc = fs->frame_acc + dt;
+    fs->iter += 1u;
+    fs->substeps += 1u;
     fs->v2max_bits = 0u;
     fs->a2max_bits = 0u;
 }

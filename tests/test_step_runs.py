@@ -26,3 +26,26 @@ def test_any_split_of_the_steps_gives_the_same_state(calls, adaptive):
                     one.advanceFrame()
                 for a, b in zip(s.getState(), one.getState()):
                     assert np.array_equal(a.view(np.uint32), b.view(np.uint32))
+
+
+@pytest.mark.parametrize("adaptive", [False, True])
+@pytest.mark.parametrize("max_substeps", [1, 4, 5, 16, 17, 21, 10000])
+@pytest.mark.parametrize("steps", [0.5, 3.5, 4.0, 5.0, 16.0, 17.5, 37.0])
+def test_a_frame_ends_where_its_sub_steps_do(steps, max_substeps, adaptive):
+    rng = np.random.default_rng(2)
+    pos = (0.1 + 0.2 * rng.random((700, 3))).astype(np.float32)
+    vel = rng.normal(scale=4.0 if adaptive else 0.5, size=pos.shape).astype(np.float32)  # CFL-limited: dt below the step
+    prm = params_16k(adaptiveTimeStep=adaptive, timeStep=2e-3)
+    frame = steps * 2e-3
+    with SPHSolver(prm) as s, SPHSolver(prm) as one:
+        s.setParticles(pos, vel)
+        one.setParticles(pos, vel)
+        for _ in range(2):
+            t, k = s.advanceFrames(1, frame, max_substeps)
+            acc, n = np.float32(0.0), 0
+            while float(acc) < frame and n < max_substeps:
+                acc = np.float32(acc + np.float32(one.advanceFrame()))
+                n += 1
+            assert k == n and np.float32(t) == acc
+            for a, b in zip(s.getState(), one.getState()):
+                assert np.array_equal(a.view(np.uint32), b.view(np.uint32))
