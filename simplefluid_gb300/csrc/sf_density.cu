@@ -129,7 +129,8 @@ void launch_density(const DeviceState& d, const SimConst& c, cudaStream_t s) {
         });
         return;
     }
-    const bool big = d.tune.density_block == 256;
+    const bool small_blocks = d.n >= kSmallBlockFrom && d.n < kSmallBlockTo && standard_passes(d);
+    const bool big = d.tune.density_block == 256 && !small_blocks;
     if (!d.nbr || d.tune.list_mode == SF_LIST_NONE) {
         big ? density_as<kEmitNone, 256>(d, c, s) : density_as<kEmitNone, 128>(d, c, s);
     } else if (d.tune.list_mode == SF_LIST_TILE_STAGED) {

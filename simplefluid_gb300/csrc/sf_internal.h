@@ -188,6 +188,12 @@ constexpr int kListedReach = 2;
 constexpr uint32_t kDensityTeamScene = 57344, kForceTeamScene = 32768;
 // Scenes from this size on launch the next pass early (allow_dependents_sized).
 constexpr uint32_t kEarlyLaunchScene = 196608;
+// Between these sizes the density pass takes blocks of 128 threads: its grid is
+// two to seven blocks of 256 per SM there, of which the last are few.  Ten
+// sub-steps, 256 / 128 threads (lattice; disordered): 76,000 particles 296 /
+// 300, 388 / 389 us; 84,000 321 / 319, 418 / 411; 120,000 456 / 432, 507 / 501;
+// 236,987 (disordered) 920 / 909; 300,000 815 / 818, 1095 / 1110.
+constexpr uint32_t kSmallBlockFrom = 81920, kSmallBlockTo = 262144;
 // Warps per 32 particles in the force pass, and neighbours they take in turn
 // (2 x 4; stage times at 16,000 and 32,000 particles 9.5 and 12.3 us, 4 x 4
 // 9.6 and 13.7, 3 x 2 9.6 and 13.9, 8 x 2 12.4 and 15.6).

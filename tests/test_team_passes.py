@@ -125,3 +125,17 @@ def test_adjoint_pairs_equal_oracle(oracle, h, seed_scale):
     want = oracle.adjoint(prm.to_c(), pos, vel, 3, gx, ckpt=2, dtype=np.float32)
     np.testing.assert_array_equal(dx0, want[0])
     np.testing.assert_array_equal(dv0, want[1])
+
+
+@pytest.mark.parametrize("n", [81919, 81920, 196607, 196608, 262143, 262144])
+def test_sizes_where_the_blocks_and_launches_change(n):
+    r = 0.0025
+    prm = params_16k(particleRadius=r, kernelRadius=4 * r)
+    pos, vel = block(n, n, spacing=2 * r)
+
+    def blocks_256(s):
+        t = s.getTuning()
+        t.density_block = t.force_block = 256
+        s.setTuning(t)
+
+    same(run(prm, pos, vel), run(prm, pos, vel, blocks_256))
