@@ -49,3 +49,20 @@ def test_a_frame_ends_where_its_sub_steps_do(steps, max_substeps, adaptive):
             assert k == n and np.float32(t) == acc
             for a, b in zip(s.getState(), one.getState()):
                 assert np.array_equal(a.view(np.uint32), b.view(np.uint32))
+
+
+@pytest.mark.parametrize("calls", [[7] * 5 + [3, 7, 9, 9, 9, 9, 7], [40] * 4 + [6], [300]])
+def test_repeated_and_long_calls_give_the_same_state(calls):
+    rng = np.random.default_rng(3)
+    pos = (0.1 + 0.3 * rng.random((900, 3))).astype(np.float32)
+    prm = params_16k(timeStep=5e-4)
+    with SPHSolver(prm) as s, SPHSolver(prm) as one:
+        for upload in (pos, pos[:800]):
+            s.setParticles(upload)
+            one.setParticles(upload)
+            for k in calls:
+                s.step(k)
+            for _ in range(sum(calls)):
+                one.advanceFrame()
+            for a, b in zip(s.getState(), one.getState()):
+                assert np.array_equal(a.view(np.uint32), b.view(np.uint32))
