@@ -286,8 +286,8 @@ typedef struct sf_tuning {
     int32_t l2_window;     /* 1: the force pass's gather records are kept in
                               L2 with a persisting access-policy window on the
                               density and force launches; 0: no window       */
-    int32_t batch_cluster; /* batches only.  0: each step is five launches
-                              over all scenes' particles.  2, 4 or 8: each step
+    int32_t batch_cluster; /* batches only.  0: each step is a launch per
+                              stage over all scenes' particles.  2, 4 or 8: each step
                               is one persistent launch of thread-block
                               clusters of that many blocks; a cluster takes
                               whole scenes, largest first, and runs their five
@@ -310,7 +310,9 @@ SF_API sf_status sf_set_tuning(sf_ctx* ctx, const sf_tuning* t);
  * of the steps; step_ms (may be NULL) receives each step's time. */
 SF_API sf_status sf_step_timed(sf_ctx* ctx, uint32_t nsteps, uint64_t flush_bytes, float* total_ms,
                                float* step_ms);
-/* Number of kernel stages in one sub-step and their names. */
+/* Number of kernel stages in one sub-step and their names.  "scatter" launches
+ * nothing where cells_per_h is 2 or more: the sort finds a cell's particles
+ * through lists there. */
 SF_API uint32_t sf_stage_count(void);
 SF_API const char* sf_stage_name(uint32_t stage);
 /* Run `nsteps` sub-steps stage by stage (no graph) with an event between

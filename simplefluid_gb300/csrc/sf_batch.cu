@@ -12,7 +12,7 @@
 // for one another: the only shared word is the queue counter (atomics), and a
 // scene's data stay in L2 across its five stages.  Every stage performs the
 // operations of the separately launched passes in the same order, so the
-// results are bit-identical to the five-kernel step.
+// results are bit-identical to the separately launched step.
 //
 // Loads of data written earlier in the same launch are plain (coherent)
 // global loads: each barrier.cluster arrive/wait pair is a release/acquire at

@@ -238,8 +238,8 @@ SF_API sf_status sf_batch_set_cells_per_h(sf_batch* b, int32_t cells_per_h) {
 }
 
 // Autotuner: times `trial_steps` graph-replayed steps (after 2 warm-up steps)
-// of every candidate configuration — grid granularity K, and either the five
-// launches' kernel variants or the persistent step's cluster and block size
+// of every candidate configuration — grid granularity K, and either the
+// separate launches' kernel variants or the persistent step's cluster and block size
 // (its partition of the scenes over the GPU) — each from the same snapshot of
 // the current state, keeps the fastest, and restores the snapshot.  The chosen K changes the summation
 // order (and so the last bits); the kernel variants do not.
@@ -259,7 +259,7 @@ SF_API sf_status sf_batch_autotune(sf_batch* b, uint32_t trial_steps, sf_tuning*
     };
     std::vector<Cand> cands;
     for (int K : {1, 2}) {
-        // five launches per step over all scenes
+        // a launch per stage over all scenes
         for (int mode : {SF_LIST_TILE_STAGED, SF_LIST_TILE, SF_LIST_TILE16})
             for (int db : {128, 256})
                 for (int fb : {128, 256}) {

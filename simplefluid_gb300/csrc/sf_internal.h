@@ -82,7 +82,7 @@ struct Tuning {
     int force_block = 128;         // 128 or 256 threads
     int prefetch = 2;              // neighbours gathered per batch in the force pass: 2 or 4
     int l2_window = 0;             // 1: persisting L2 window over the gather records
-    int batch_cluster = 0;         // batches: 0 five launches per step; 2, 4, 8 one persistent launch of clusters
+    int batch_cluster = 0;         // batches: 0 a launch per stage; 2, 4, 8 one persistent launch of clusters
     int batch_block = 0;           // threads per block of the persistent step: 256, 512, 1024 (0: 256)
 };
 
