@@ -71,6 +71,8 @@ struct sf_ctx {
     cudaGraphExec_t run_graph = nullptr;   // kRunSteps sub-steps
     cudaGraphExec_t call_graph = nullptr;  // call_steps sub-steps
     uint32_t call_steps = 0, last_steps = 0, repeats = 0;  // the last call's sub-steps, and how often they repeated
+    uint64_t stepped_at = 0;               // see note_sharing
+    uint32_t sharing_calls = 0;
     bool stepped = false;                  // a call stepped since the graphs were last dropped
     bool sorted = false;  // particles uploaded and cell-sorted
     float* h_stage = nullptr;  // pinned staging for pageable caller buffers

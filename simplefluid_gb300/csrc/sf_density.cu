@@ -121,7 +121,7 @@ bool standard_passes(const DeviceState& d) {
 
 void launch_density(const DeviceState& d, const SimConst& c, cudaStream_t s) {
     if (!d.n) return;
-    if (d.n < kDensityTeamScene && standard_passes(d)) {
+    if (d.n < kDensityTeamScene && !d.shared && standard_passes(d)) {
         with_reach(c.reach, [&](auto R) {
             constexpr int K = decltype(R)::value;
             launch_chained(k_density_team<K>, grid_for(d.n, kTeamParticles), (2 * K + 1) * 32, s, d.pos, d.cell_start,

@@ -150,7 +150,7 @@ void force_as(DeviceState& d, const SimConst& c, cudaStream_t s) {
 template <bool kIntegrate>
 void launch_force(DeviceState& d, const SimConst& c, cudaStream_t s) {
     if (!d.n) return;
-    if (d.n < kForceTeamScene && standard_passes(d)) {
+    if (d.n < kForceTeamScene && !d.shared && standard_passes(d)) {
         force_team_as<kIntegrate, kForceTeam, kForceTurn>(d, c, s);
         return;
     }

@@ -105,6 +105,7 @@ struct DeviceState {
     uint8_t* nbr_wide = nullptr;   // SF_LIST_TILE16: per warp tile (kNbWarpTile particles), 1 where it holds 32-bit entries
     float4* pv = nullptr;          // 2 per particle (32 bytes): (x, vx, y, vy), (z, vz, p, 1/rho)
     float4* sums = nullptr;        // optional: per particle (AP, 0), (AV, 0) of the force pass (adjoint recording)
+    bool shared = false;           // other contexts step on the GPU in between: no team passes
     FrameState* frame = nullptr;   // adaptive sub-steps read dt here and raise the maxima
     // grid
     uint32_t ncells = 0, ncells_pad = 0;

@@ -66,3 +66,32 @@ def test_repeated_and_long_calls_give_the_same_state(calls):
                 one.advanceFrame()
             for a, b in zip(s.getState(), one.getState()):
                 assert np.array_equal(a.view(np.uint32), b.view(np.uint32))
+
+
+def test_contexts_stepped_in_turn_give_the_state_of_one_alone():
+    """Four small scenes and the calls that decide whether they share the GPU."""
+    rng = np.random.default_rng(4)
+    prm = params_16k(particleRadius=0.005, kernelRadius=0.02)
+    pos = [(0.05 + 0.35 * rng.random((25000, 3))).astype(np.float32) for _ in range(4)]
+    alone = []
+    for p in pos:
+        with SPHSolver(prm) as s:
+            s.setParticles(p)
+            s.step(14)
+            alone.append(s.getState())
+    solvers = [SPHSolver(prm) for _ in pos]
+    try:
+        for s, p in zip(solvers, pos):
+            s.setParticles(p)
+        for _ in range(9):  # in turn: from the fifth round on as sharing
+            for s in solvers:
+                s.step(1)
+        for s in solvers:  # each by itself again
+            for _ in range(5):
+                s.step(1)
+        for s, want in zip(solvers, alone):
+            for a, b in zip(s.getState(), want):
+                assert np.array_equal(a.view(np.uint32), b.view(np.uint32))
+    finally:
+        for s in solvers:
+            s.close()
