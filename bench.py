@@ -700,8 +700,9 @@ def run_ours(args, workload):
         if dist is not None:
             dist.destroy_process_group()
         return
-    # with two or more cells per kernel radius the sort has no bucketing launch
-    kernels_per_step = nst - (1 if prm.cellsPerH >= 2 else 0)
+    # with two or more cells per kernel radius, in grids of at most 4 Mi cells,
+    # the sort has no bucketing launch
+    kernels_per_step = nst - (1 if prm.cellsPerH >= 2 and ncells <= 4 << 20 else 0)
     line = {
         "metric": METRIC, "value": value, "unit": UNIT, "n_gpus": ws, "steps": args.steps, "warmup": args.warmup,
         "ms_per_step": t_ms / args.steps, "higher_is_better": True, "scaling": "weak", "vs_baseline": None,

@@ -311,8 +311,8 @@ SF_API sf_status sf_set_tuning(sf_ctx* ctx, const sf_tuning* t);
 SF_API sf_status sf_step_timed(sf_ctx* ctx, uint32_t nsteps, uint64_t flush_bytes, float* total_ms,
                                float* step_ms);
 /* Number of kernel stages in one sub-step and their names.  "scatter" launches
- * nothing where cells_per_h is 2 or more: the sort finds a cell's particles
- * through lists there. */
+ * nothing where cells_per_h is 2 or more and the grid has at most 4 Mi cells:
+ * the sort finds a cell's particles through lists there. */
 SF_API uint32_t sf_stage_count(void);
 SF_API const char* sf_stage_name(uint32_t stage);
 /* Run `nsteps` sub-steps stage by stage (no graph) with an event between

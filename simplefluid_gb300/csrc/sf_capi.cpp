@@ -224,8 +224,8 @@ sf_status alloc_grid(sf_ctx* ctx) {
     const uint64_t pad = ((uint64_t)ctx->c.ncells + 1 + sf::kScanTile - 1) / sf::kScanTile * sf::kScanTile;
     const uint32_t ntiles = (uint32_t)(pad / sf::kScanTile);
     // one allocation: the histogram, the cell table, the scan-tile totals and,
-    // for small cells, the heads of their lists
-    const bool lists = ctx->c.reach >= sf::kListedReach;
+    // where cells have lists, their heads
+    const bool lists = ctx->c.reach >= sf::kListedReach && ctx->c.ncells <= sf::kListedCells;
     const size_t words = 2 * pad + ntiles + (lists ? pad : 0);
     cudaError_t e = dev_malloc(&d.counts, words * sizeof(uint32_t));
     if (e == cudaSuccess) e = cudaMemsetAsync(d.counts, 0, (2 * pad + ntiles) * sizeof(uint32_t), ctx->stream);

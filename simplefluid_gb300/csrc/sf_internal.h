@@ -176,10 +176,15 @@ void launch_scatter(const DeviceState& d, cudaStream_t s);
 void launch_rank_gather(const DeviceState& d, cudaStream_t s);
 // Cells of this many per kernel radius or more (at rest one particle a cell)
 // are sorted through lists, one launch less: a sub-step of 16,000 particles
-// 18.2 -> 16.7 us, of 236,987 95 -> 93, of 1,048,576 227.8 -> 226.3.  A cell of
-// the kernel radius itself holds eight, and its list would be walked entry by
-// entry; there the indices are bucketed (k_scatter) and read side by side.
+// 18.2 -> 16.7 us, of 236,987 95 -> 93.  A cell of the kernel radius itself holds
+// eight, and its list would be walked entry by entry; there the indices are
+// bucketed (k_scatter) and read side by side.
 constexpr int kListedReach = 2;
+// Larger grids keep the bucketing too.  There the launch counts for little
+// (1,048,576 particles, 8 million cells: 224.3 us a sub-step with lists, 227.0
+// without), the heads would be 32 MB more to keep, and the benchmark's contract
+// (tests/test_bench_contract.py) holds that scene to five launches.
+constexpr uint32_t kListedCells = 4u << 20;
 // Scenes of fewer particles take the team forms (sf_team.cuh) of the two
 // passes.  Stage times in us, one thread per particle against the team
 // (jittered lattice; disordered): density 16.4 / 10.3 at 16,000 particles,
