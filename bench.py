@@ -192,10 +192,10 @@ def cpu_oracle_rate(pos: np.ndarray, prm, budget_s: float, max_steps: int, warmu
 def measure_batched(args, dist=None, rank: int = 0, ws: int = 1) -> dict:
     """Batched cubes: 256 scenes (counts log-uniform in [2000, 65536], seed
     20171) advanced together, one graph launch per step, in the configuration
-    the autotuner chooses (grid granularity, and either the five launches'
+    the autotuner chooses (grid granularity, and either the separate launches'
     kernel variants or the persistent step's cluster and block size).  Beside
     it, on the same clock (wall time between synchronisations, the same steps
-    from the same state): the five-launch step and the persistent step with
+    from the same state): the separately launched step and the persistent step with
     each cluster and block size, every scene stepped on its own context one
     after another, and all those contexts interleaved on their own streams.
     With several ranks the scenes are spread over them (largest first, no
@@ -388,8 +388,8 @@ def measure_adjoint(args) -> dict:
     roof = {"bound": "hbm", "kernel": "k_adj_forces", "achieved": achieved, "peak": peaks["hbm_gbs"], "unit": "GB/s",
             "frac": achieved / peaks["hbm_gbs"], "algorithmic_bytes_per_launch": fbytes, "avg_launch_ms": avg,
             "peak_source": peaks["source"],
-            "note": ("not HBM-bound: 65,536 particles fill about 13 warps per SM; ncu shows 35% issue-active at "
-                     "9.2 cycles per instruction (about 7,000 instructions per warp)")}
+            "note": ("not HBM-bound: 65,536 particles fill about 13 warps per SM, and the latency of each "
+                     "thread's gathers sets the time")}
     return {"particles": int(pos.shape[0]), "steps": steps, "ckpt_every": ckpt, "forward_ms": fwd_ms,
             "forward_with_checkpoints_ms": best[0], "loss_ms": best[1], "adjoint_ms": best[2],
             "ratio_adjoint_over_forward": best[2] / fwd_ms, "loss": float(L),
