@@ -206,11 +206,33 @@ void free_render(sf_ctx* ctx) {
     ctx->render_n = 0;
 }
 
+static void destroy_retired(sf_ctx* ctx) {
+    for (uint32_t k = 0; k < ctx->nretired; ++k) cudaGraphExecDestroy(ctx->retired[k]);
+    ctx->nretired = 0;
+}
+
+// No graph is destroyed while its launches are queued or running: a program
+// that steps many contexts without waiting for them has long queues of them.
+void retire_graph(sf_ctx* ctx, cudaGraphExec_t& g) {
+    if (!g) return;
+    if (ctx->nretired == sizeof(ctx->retired) / sizeof(ctx->retired[0])) {
+        cudaStreamSynchronize(ctx->stream);
+        destroy_retired(ctx);
+    }
+    ctx->retired[ctx->nretired++] = g;
+    g = nullptr;
+}
+
+sf_status wait_stream(sf_ctx* ctx) {
+    SF_CUDA(cudaStreamSynchronize(ctx->stream));
+    destroy_retired(ctx);
+    return SF_OK;
+}
+
 void drop_graph(sf_ctx* ctx) {
-    if (ctx->step_graph) cudaGraphExecDestroy(ctx->step_graph);
-    if (ctx->run_graph) cudaGraphExecDestroy(ctx->run_graph);
-    if (ctx->call_graph) cudaGraphExecDestroy(ctx->call_graph);
-    ctx->step_graph = ctx->run_graph = ctx->call_graph = nullptr;
+    retire_graph(ctx, ctx->step_graph);
+    retire_graph(ctx, ctx->run_graph);
+    retire_graph(ctx, ctx->call_graph);
     ctx->call_steps = ctx->last_steps = ctx->repeats = 0;
     ctx->stepped = false;
     ++ctx->gen;
@@ -371,7 +393,8 @@ sf_status capture_steps(sf_ctx* ctx, uint32_t nsteps, cudaGraphExec_t* out) {
 // GPU drains.  20 sub-steps of 16,000 particles 393 -> 376 us, of 65,536
 // 852 -> 827, 10 of 236,987 973 -> 953, of 1,048,576 2314 -> 2285.
 constexpr uint32_t kRunSteps = 5;
-// A first call of at most this many sub-steps queues the kernels themselves:
+// A first call of at most this many sub-steps queues the kernels themselves
+// (a later one's last few go through the graph of one sub-step):
 // that takes the host less time than making a graph (20 sub-steps of 16,000
 // particles on a new context 640 -> 580 us), and a context may step only once.
 constexpr uint32_t kFirstSteps = 32;
@@ -388,8 +411,7 @@ static sf_status need_call_graph(sf_ctx* ctx, uint32_t nsteps) {
     ctx->last_steps = nsteps;
     const uint32_t len = std::min(nsteps, kCallSteps);
     if (len <= kRunSteps || len == ctx->call_steps || (ctx->repeats < 2 && nsteps < kLongCall)) return SF_OK;
-    if (ctx->call_graph) cudaGraphExecDestroy(ctx->call_graph);
-    ctx->call_graph = nullptr;
+    retire_graph(ctx, ctx->call_graph);
     ctx->call_steps = 0;
     SF_TRY(capture_steps(ctx, len, &ctx->call_graph));
     ctx->call_steps = len;
@@ -416,6 +438,7 @@ static void note_sharing(sf_ctx* ctx) {
     } else if (++ctx->sharing_calls == 4) {
         ctx->sharing_calls = 0;
         drop_graph(ctx);
+        ctx->stepped = true;  // graphs again at once: kernels are queued directly behind uploads only
         ctx->d.shared = shared;
     }
 }
@@ -434,8 +457,7 @@ sf_status launch_steps(sf_ctx* ctx, uint32_t nsteps) {
         for (; left >= kRunSteps; left -= kRunSteps) SF_CUDA(cudaGraphLaunch(ctx->run_graph, ctx->stream));
     }
     if (!left) return SF_OK;
-    if (!graphs || (nsteps >= kRunSteps && !ctx->step_graph)) {
-        // a call's few last sub-steps are not worth a graph of their own either
+    if (!graphs) {
         for (; left; --left) enqueue_full_step(ctx);
         return check_launch("step");
     }
@@ -460,12 +482,12 @@ sf_status copy_out(sf_ctx* ctx, void* dst, const void* src, size_t bytes) {
     if (!bytes) return SF_OK;
     if (is_pinned(dst)) {
         SF_CUDA(cudaMemcpyAsync(dst, src, bytes, cudaMemcpyDeviceToHost, ctx->stream));
-        SF_CUDA(cudaStreamSynchronize(ctx->stream));
+        SF_TRY(wait_stream(ctx));
         return SF_OK;
     }
     SF_TRY(ensure_stage(ctx, bytes));
     SF_CUDA(cudaMemcpyAsync(ctx->h_stage, src, bytes, cudaMemcpyDeviceToHost, ctx->stream));
-    SF_CUDA(cudaStreamSynchronize(ctx->stream));
+    SF_TRY(wait_stream(ctx));
     std::memcpy(dst, ctx->h_stage, bytes);
     return SF_OK;
 }
@@ -477,7 +499,7 @@ sf_status copy_in(sf_ctx* ctx, void* dst, const void* src, size_t bytes) {
         return SF_OK;
     }
     SF_TRY(ensure_stage(ctx, bytes));
-    SF_CUDA(cudaStreamSynchronize(ctx->stream));  // staging may still feed an earlier copy
+    SF_TRY(wait_stream(ctx));  // staging may still feed an earlier copy
     std::memcpy(ctx->h_stage, src, bytes);
     SF_CUDA(cudaMemcpyAsync(dst, ctx->h_stage, bytes, cudaMemcpyHostToDevice, ctx->stream));
     return SF_OK;
@@ -504,11 +526,11 @@ void release_ctx(sf_ctx* ctx) {
     if (ctx->aux) cudaStreamSynchronize(ctx->aux);
     free_trajectory(ctx);
     free_render(ctx);
-    if (ctx->frame_graph) cudaGraphExecDestroy(ctx->frame_graph);
-    ctx->frame_graph = nullptr;
+    retire_graph(ctx, ctx->frame_graph);
     if (ctx->frame) cudaFree(ctx->frame);
     ctx->frame = nullptr;
     drop_graph(ctx);
+    destroy_retired(ctx);
     free_particles(ctx->d);
     free_grid(ctx->d);
     if (ctx->h_stage) cudaFreeHost(ctx->h_stage);
@@ -790,7 +812,7 @@ SF_API sf_status sf_set_params(sf_ctx* ctx, const sf_params* p) {
     const int st = sf::derive_constants(*p, &c, &why);
     if (st) return fail(st, why);
     SF_TRY(set_device(ctx));
-    SF_CUDA(cudaStreamSynchronize(ctx->stream));
+    SF_TRY(wait_stream(ctx));
     const bool grid_changed = std::memcmp(c.n, ctx->c.n, sizeof(c.n)) != 0 ||
                               std::memcmp(c.bmin, ctx->c.bmin, sizeof(c.bmin)) != 0 ||
                               std::memcmp(c.inv_cell, ctx->c.inv_cell, sizeof(c.inv_cell)) != 0;
@@ -845,7 +867,7 @@ SF_API sf_status sf_set_state(sf_ctx* ctx, const float* pos_xyz, const float* ve
     if (host_direct(ctx, pos_xyz) && (!vel_xyz || host_direct(ctx, vel_xyz))) {
         // pageable arrays the GPU reads in place: no staging copy
         SF_TRY(sort_uploaded(ctx, pos_xyz, vel_xyz));
-        SF_CUDA(cudaStreamSynchronize(ctx->stream));
+        SF_TRY(wait_stream(ctx));
         return SF_OK;
     }
     float* io = ctx->d.io;
@@ -854,7 +876,7 @@ SF_API sf_status sf_set_state(sf_ctx* ctx, const float* pos_xyz, const float* ve
     if (vel_xyz) SF_TRY(copy_in(ctx, io + 3 * (size_t)n, vel_xyz, bytes));
     SF_TRY(sort_uploaded(ctx, io, vel_xyz ? io + 3 * (size_t)n : nullptr));
     // The caller may reuse its buffers once this returns.
-    SF_CUDA(cudaStreamSynchronize(ctx->stream));
+    SF_TRY(wait_stream(ctx));
     return SF_OK;
 }
 
@@ -869,7 +891,7 @@ SF_API sf_status sf_get_state(sf_ctx* ctx, float* pos_xyz, float* vel_xyz, uint3
         populate_pages(vel_xyz, (size_t)n * 3 * sizeof(float));
         sf::launch_store_caller_order(ctx->d.pos, ctx->d.vel, n, ctx->d.tmp, pos_xyz, vel_xyz, ctx->stream);
         SF_TRY(check_launch("store state"));
-        SF_CUDA(cudaStreamSynchronize(ctx->stream));
+        SF_TRY(wait_stream(ctx));
         return SF_OK;
     }
     float* io = ctx->d.io;
@@ -887,7 +909,7 @@ SF_API sf_status sf_get_state(sf_ctx* ctx, float* pos_xyz, float* vel_xyz, uint3
         SF_CUDA(cudaMemcpyAsync(vel_xyz, io + 3 * (size_t)n, bytes, cudaMemcpyDeviceToHost, ctx->aux));
         SF_CUDA(cudaEventRecord(ctx->ev_out, ctx->aux));
         SF_CUDA(cudaStreamWaitEvent(ctx->stream, ctx->ev_out, 0));  // later work waits for the velocity reads
-        SF_CUDA(cudaStreamSynchronize(ctx->stream));
+        SF_TRY(wait_stream(ctx));
         return SF_OK;
     }
     sf::launch_store_aos(ctx->d.pos, ctx->d.vel, n, pos_xyz ? io : nullptr, vel_xyz ? io + 3 * (size_t)n : nullptr,
@@ -898,12 +920,12 @@ SF_API sf_status sf_get_state(sf_ctx* ctx, float* pos_xyz, float* vel_xyz, uint3
         if (pos_xyz) SF_CUDA(cudaMemcpyAsync(pos_xyz, io, bytes, cudaMemcpyDeviceToHost, ctx->stream));
         if (vel_xyz)
             SF_CUDA(cudaMemcpyAsync(vel_xyz, io + 3 * (size_t)n, bytes, cudaMemcpyDeviceToHost, ctx->stream));
-        SF_CUDA(cudaStreamSynchronize(ctx->stream));
+        SF_TRY(wait_stream(ctx));
         return SF_OK;
     }
     if (pos_xyz) SF_TRY(copy_out(ctx, pos_xyz, io, bytes));
     if (vel_xyz) SF_TRY(copy_out(ctx, vel_xyz, io + 3 * (size_t)n, bytes));
-    SF_CUDA(cudaStreamSynchronize(ctx->stream));
+    SF_TRY(wait_stream(ctx));
     return SF_OK;
 }
 
@@ -1004,7 +1026,7 @@ SF_API sf_status sf_advance_frame(sf_ctx* ctx, float* dt_out) {
         return SF_OK;
     }
     SF_CUDA(cudaMemcpyAsync(dt_out, &ctx->frame->dt, sizeof(float), cudaMemcpyDeviceToHost, ctx->stream));
-    SF_CUDA(cudaStreamSynchronize(ctx->stream));
+    SF_TRY(wait_stream(ctx));
     return SF_OK;
 }
 
@@ -1075,8 +1097,7 @@ SF_API sf_status sf_advance_frames(sf_ctx* ctx, uint32_t frames, double frame_ti
     if (!(frame_time > 0.0) || max_substeps == 0) return fail(SF_ERR_INVALID_ARGUMENT, "need frame_time > 0, max_substeps > 0");
     if (!ctx->frame_graph || ctx->frame_graph_gen != ctx->gen || ctx->frame_graph_time != frame_time ||
         ctx->frame_graph_max != max_substeps) {
-        if (ctx->frame_graph) cudaGraphExecDestroy(ctx->frame_graph);
-        ctx->frame_graph = nullptr;
+        retire_graph(ctx, ctx->frame_graph);
         SF_TRY(build_frame_graph(ctx, frame_time, max_substeps, &ctx->frame_graph));
         ctx->frame_graph_gen = ctx->gen;
         ctx->frame_graph_time = frame_time;
@@ -1087,7 +1108,7 @@ SF_API sf_status sf_advance_frames(sf_ctx* ctx, uint32_t frames, double frame_ti
     for (uint32_t f = 0; f < frames; ++f) SF_CUDA(cudaGraphLaunch(ctx->frame_graph, ctx->stream));
     sf::FrameState fs;
     SF_CUDA(cudaMemcpyAsync(&fs, ctx->frame, sizeof(fs), cudaMemcpyDeviceToHost, ctx->stream));
-    SF_CUDA(cudaStreamSynchronize(ctx->stream));
+    SF_TRY(wait_stream(ctx));
     if (sim_time_out) *sim_time_out = fs.sim_time;
     if (substeps_out) *substeps_out = fs.substeps;
     return SF_OK;
@@ -1103,7 +1124,7 @@ SF_API sf_status sf_step(sf_ctx* ctx, uint32_t nsteps) {
 SF_API sf_status sf_synchronize(sf_ctx* ctx) {
     SF_TRY(need_ctx(ctx));
     SF_TRY(set_device(ctx));
-    SF_CUDA(cudaStreamSynchronize(ctx->stream));
+    SF_TRY(wait_stream(ctx));
     return SF_OK;
 }
 

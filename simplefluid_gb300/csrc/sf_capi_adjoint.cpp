@@ -79,7 +79,7 @@ sf_status upload_by_id(sf_ctx* ctx, float4* dst, const float* src_xyz) {
         h[i] = src_xyz ? make_float4(src_xyz[3 * (size_t)i], src_xyz[3 * (size_t)i + 1], src_xyz[3 * (size_t)i + 2], 0.f)
                        : make_float4(0.f, 0.f, 0.f, 0.f);
     SF_CUDA(cudaMemcpyAsync(dst, h.data(), (size_t)n * sizeof(float4), cudaMemcpyHostToDevice, ctx->stream));
-    SF_CUDA(cudaStreamSynchronize(ctx->stream));
+    SF_TRY(wait_stream(ctx));
     return SF_OK;
 }
 
@@ -302,7 +302,7 @@ SF_API sf_status sf_adjoint(sf_ctx* ctx, const float* dloss_dx, const float* dlo
     if (dloss_dviscosity) *dloss_dviscosity = (float)(sc[0] * (mass * 45.0 / (kPi * h6)));
     if (dloss_dstiffness) *dloss_dstiffness = (float)sc[1];
     SF_TRY(restore_sorted(ctx, t->snap));
-    SF_CUDA(cudaStreamSynchronize(ctx->stream));
+    SF_TRY(wait_stream(ctx));
     return SF_OK;
 }
 

@@ -40,7 +40,7 @@ sf_status batch_upload_table(sf_batch* b) {
     if (!b->d_table) SF_CUDA(dev_malloc(&b->d_table, ns * sizeof(sf::SimConst)));
     SF_CUDA(cudaMemcpyAsync(b->d_table, b->consts.data(), ns * sizeof(sf::SimConst), cudaMemcpyHostToDevice,
                             b->eng.stream));
-    SF_CUDA(cudaStreamSynchronize(b->eng.stream));
+    SF_TRY(wait_stream(&b->eng));
     b->eng.d.table = b->d_table;
     b->eng.d.scene_off = b->d_off;
     b->eng.d.nscenes = (uint32_t)ns;
@@ -160,7 +160,7 @@ SF_API sf_status sf_batch_set_state(sf_batch* b, const uint32_t* counts, const f
         off[s + 1] = (uint32_t)next;
     }
     SF_TRY(set_device(&b->eng));
-    SF_CUDA(cudaStreamSynchronize(b->eng.stream));
+    SF_TRY(wait_stream(&b->eng));
     SF_CUDA(cudaMemcpy(b->d_off, off.data(), off.size() * sizeof(uint32_t), cudaMemcpyHostToDevice));
     // the persistent step's queue order: largest scenes first (ties by index)
     std::vector<uint32_t> order(ns);
@@ -220,7 +220,7 @@ SF_API sf_status sf_batch_set_cells_per_h(sf_batch* b, int32_t cells_per_h) {
     SF_TRY(need_batch(b));
     if (cells_per_h != 1 && cells_per_h != 2) return fail(SF_ERR_INVALID_ARGUMENT, "batches support cells_per_h 1 or 2");
     SF_TRY(set_device(&b->eng));
-    SF_CUDA(cudaStreamSynchronize(b->eng.stream));
+    SF_TRY(wait_stream(&b->eng));
     SF_TRY(batch_derive(b, cells_per_h));
     drop_graph(&b->eng);
     SF_TRY(alloc_grid(&b->eng));

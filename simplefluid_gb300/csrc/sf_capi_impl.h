@@ -70,6 +70,10 @@ struct sf_ctx {
     cudaGraphExec_t step_graph = nullptr;  // one sub-step
     cudaGraphExec_t run_graph = nullptr;   // kRunSteps sub-steps
     cudaGraphExec_t call_graph = nullptr;  // call_steps sub-steps
+    // graphs given up while queued work may still use them: destroyed after a
+    // wait for the stream
+    cudaGraphExec_t retired[8] = {};
+    uint32_t nretired = 0;
     uint32_t call_steps = 0, last_steps = 0, repeats = 0;  // the last call's sub-steps, and how often they repeated
     uint64_t stepped_at = 0;               // see note_sharing
     uint32_t sharing_calls = 0;
@@ -164,6 +168,10 @@ void enqueue_full_step(sf_ctx* ctx);
 sf_status capture_steps(sf_ctx* ctx, uint32_t nsteps, cudaGraphExec_t* out);
 sf_status launch_steps(sf_ctx* ctx, uint32_t nsteps);
 void drop_graph(sf_ctx* ctx);
+// Gives up a graph that may be queued or running.
+void retire_graph(sf_ctx* ctx, cudaGraphExec_t& g);
+// Waits for the context's stream.
+sf_status wait_stream(sf_ctx* ctx);
 // Kernel choices by particle count, unless the caller set them explicitly.
 void apply_size_defaults(sf_ctx* ctx);
 

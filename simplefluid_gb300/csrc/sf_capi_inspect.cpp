@@ -58,7 +58,7 @@ SF_API sf_status sf_compute_density(sf_ctx* ctx, float* rho, float* pressure, ui
         SF_TRY(copy_out(ctx, pr.data(), ctx->d.pr, (size_t)n * sizeof(float2)));
         for (uint32_t i = 0; i < n; ++i) pressure[i] = pr[i].x;
     }
-    SF_CUDA(cudaStreamSynchronize(ctx->stream));
+    SF_TRY(wait_stream(ctx));
     return SF_OK;
 }
 
@@ -125,7 +125,7 @@ SF_API sf_status sf_check_state(sf_ctx* ctx, sf_state_report* report) {
     SF_TRY(check_launch("check state"));
     uint32_t r[sf::kReportWords];
     SF_CUDA(cudaMemcpyAsync(r, ctx->d_report, sizeof(r), cudaMemcpyDeviceToHost, ctx->stream));
-    SF_CUDA(cudaStreamSynchronize(ctx->stream));
+    SF_TRY(wait_stream(ctx));
     report->n = ctx->d.n;
     report->non_finite = r[0];
     report->outside_box = r[1];
@@ -182,7 +182,7 @@ SF_API sf_status sf_step_timed(sf_ctx* ctx, uint32_t nsteps, uint64_t flush_byte
         SF_CUDA(cudaGraphLaunch(ctx->step_graph, ctx->stream));
         SF_CUDA(cudaEventRecord(ev.ev[2 * i + 1], ctx->stream));
     }
-    SF_CUDA(cudaStreamSynchronize(ctx->stream));
+    SF_TRY(wait_stream(ctx));
     double total = 0.0;
     for (uint32_t i = 0; i < nsteps; ++i) {
         float ms = 0.f;
@@ -227,7 +227,7 @@ SF_API sf_status sf_set_tuning(sf_ctx* ctx, const sf_tuning* t) {
     if (t->prefetch != 2 && t->prefetch != 4) return fail(SF_ERR_INVALID_ARGUMENT, "prefetch must be 2 or 4");
     if (t->reserved[0]) return fail(SF_ERR_INVALID_ARGUMENT, "reserved fields must be zero");
     SF_TRY(set_device(ctx));
-    SF_CUDA(cudaStreamSynchronize(ctx->stream));
+    SF_TRY(wait_stream(ctx));
     ctx->d.tune.list_mode = t->list_mode;
     ctx->d.tune.density_block = t->density_block;
     ctx->d.tune.force_block = t->force_block;
@@ -265,7 +265,7 @@ SF_API sf_status sf_profile_steps(sf_ctx* ctx, uint32_t nsteps, uint64_t flush_b
         }
     }
     SF_TRY(check_launch("profiled step"));
-    SF_CUDA(cudaStreamSynchronize(ctx->stream));
+    SF_TRY(wait_stream(ctx));
     std::vector<double> acc(sf::kNumStages, 0.0);
     for (uint32_t i = 0; i < nsteps; ++i)
         for (uint32_t s = 0; s < sf::kNumStages; ++s) {
@@ -318,7 +318,7 @@ SF_API sf_status sf_adjoint_profile(sf_ctx* ctx, float* pass_ms, uint32_t npasse
         }
     }
     SF_TRY(check_launch("profiled adjoint"));
-    SF_CUDA(cudaStreamSynchronize(ctx->stream));
+    SF_TRY(wait_stream(ctx));
     for (uint32_t k = 0; k < len; ++k)
         for (uint32_t p = 0; p < sf::kAdjointPasses; ++p) {
             float ms = 0.f;
@@ -417,7 +417,7 @@ SF_API sf_status sf_render(sf_ctx* ctx, const sf_render_params* rp, float* rgba_
     if (rgba_out) SF_TRY(copy_out(ctx, rgba_out, ctx->render_rgba, np * sizeof(float4)));
     if (depth_out) SF_TRY(copy_out(ctx, depth_out, ctx->render_depth, np * sizeof(float)));
     if (owner_out) SF_TRY(copy_out(ctx, owner_out, ctx->render_owner, np * sizeof(uint32_t)));
-    SF_CUDA(cudaStreamSynchronize(ctx->stream));
+    SF_TRY(wait_stream(ctx));
     return SF_OK;
 }
 
@@ -499,7 +499,7 @@ SF_API sf_status sf_load_state(sf_ctx* ctx, const char* path, double* sim_time_o
         sf::enqueue_sort_tail(d, ctx->stream);
         if (ctx->c.adaptive) sf::launch_init_maxima(d.vel, n, ctx->frame, ctx->stream);
         SF_TRY(check_launch("load state"));
-        SF_CUDA(cudaStreamSynchronize(ctx->stream));
+        SF_TRY(wait_stream(ctx));
         ctx->sorted = true;
     }
     if (sim_time_out) *sim_time_out = t;
