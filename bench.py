@@ -617,6 +617,7 @@ def run_ours(args, workload):
     stage_ms = np.zeros(nst, np.float32)
     C.check(lib.sf_profile_steps(ctx, args.steps, FLUSH_BYTES, stage_ms.ctypes.data_as(ctypes.c_void_p), nst))
     names = [lib.sf_stage_name(i).decode() for i in range(nst)]
+    kernels_per_step = sum(1 for k in solver.stageKernels().values() if k)
     avg_ms = {nm: float(stage_ms[i]) / args.steps for i, nm in enumerate(names)}
     dom = max(avg_ms, key=avg_ms.get)
     nx, ny, nz = solver.gridDims()
@@ -700,9 +701,6 @@ def run_ours(args, workload):
         if dist is not None:
             dist.destroy_process_group()
         return
-    # with two or more cells per kernel radius, in grids of at most 4 Mi cells,
-    # the sort has no bucketing launch
-    kernels_per_step = nst - (1 if prm.cellsPerH >= 2 and ncells <= 4 << 20 else 0)
     line = {
         "metric": METRIC, "value": value, "unit": UNIT, "n_gpus": ws, "steps": args.steps, "warmup": args.warmup,
         "ms_per_step": t_ms / args.steps, "higher_is_better": True, "scaling": "weak", "vs_baseline": None,

@@ -310,11 +310,14 @@ SF_API sf_status sf_set_tuning(sf_ctx* ctx, const sf_tuning* t);
  * of the steps; step_ms (may be NULL) receives each step's time. */
 SF_API sf_status sf_step_timed(sf_ctx* ctx, uint32_t nsteps, uint64_t flush_bytes, float* total_ms,
                                float* step_ms);
-/* Number of kernel stages in one sub-step and their names.  "scatter" launches
- * nothing where cells_per_h is 2 or more and the grid has at most 4 Mi cells:
- * the sort finds a cell's particles through lists there. */
+/* Number of kernel stages in one sub-step and their names. */
 SF_API uint32_t sf_stage_count(void);
 SF_API const char* sf_stage_name(uint32_t stage);
+/* The kernel that the stage launches for the context's current state and
+ * choices, as a static string; "" where it launches none (as "scatter" does
+ * where the sort finds a cell's particles through lists).  The stages with a
+ * name are the launches of a sub-step. */
+SF_API const char* sf_stage_kernel(const sf_ctx* ctx, uint32_t stage);
 /* Run `nsteps` sub-steps stage by stage (no graph) with an event between
  * stages; stage_ms[s] receives the summed device time of stage s over all
  * steps (nstages must equal sf_stage_count()). */

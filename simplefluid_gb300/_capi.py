@@ -171,6 +171,7 @@ PROTOTYPES = {
     "sf_step_timed": (c_int32, [c_void_p, c_uint32, c_uint64, _P(c_float), c_void_p]),
     "sf_stage_count": (c_uint32, []),
     "sf_stage_name": (c_char_p, [c_uint32]),
+    "sf_stage_kernel": (c_char_p, [c_void_p, c_uint32]),
     "sf_profile_steps": (c_int32, [c_void_p, c_uint32, c_uint64, c_void_p, c_uint32]),
     "sf_adjoint_pass_count": (c_uint32, []),
     "sf_adjoint_pass_name": (c_char_p, [c_uint32]),

@@ -119,9 +119,23 @@ bool standard_passes(const DeviceState& d) {
            !d.tune.l2_window;
 }
 
+// The density pass's form: threads per block, or 0 for the team.
+static int density_form(const DeviceState& d) {
+    if (d.n < kDensityTeamScene && !d.shared && standard_passes(d)) return 0;
+    if (d.n >= kSmallBlockFrom && d.n < kSmallBlockTo && standard_passes(d)) return 128;
+    if (d.nbr && d.tune.list_mode == SF_LIST_TILE_STAGED) return kNbTile;
+    return d.tune.density_block;
+}
+
+const char* density_kernel(const DeviceState& d) {
+    const int form = density_form(d);
+    return form == 0 ? "density_team" : form == 128 ? "density_128" : "density_256";
+}
+
 void launch_density(const DeviceState& d, const SimConst& c, cudaStream_t s) {
     if (!d.n) return;
-    if (d.n < kDensityTeamScene && !d.shared && standard_passes(d)) {
+    const int form = density_form(d);
+    if (form == 0) {
         with_reach(c.reach, [&](auto R) {
             constexpr int K = decltype(R)::value;
             launch_chained(k_density_team<K>, grid_for(d.n, kTeamParticles), (2 * K + 1) * 32, s, d.pos, d.cell_start,
@@ -129,8 +143,7 @@ void launch_density(const DeviceState& d, const SimConst& c, cudaStream_t s) {
         });
         return;
     }
-    const bool small_blocks = d.n >= kSmallBlockFrom && d.n < kSmallBlockTo && standard_passes(d);
-    const bool big = d.tune.density_block == 256 && !small_blocks;
+    const bool big = form == 256;
     if (!d.nbr || d.tune.list_mode == SF_LIST_NONE) {
         big ? density_as<kEmitNone, 256>(d, c, s) : density_as<kEmitNone, 128>(d, c, s);
     } else if (d.tune.list_mode == SF_LIST_TILE_STAGED) {

@@ -147,10 +147,12 @@ void force_as(DeviceState& d, const SimConst& c, cudaStream_t s) {
     });
 }
 
+bool team_force(const DeviceState& d) { return d.n < kForceTeamScene && !d.shared && standard_passes(d); }
+
 template <bool kIntegrate>
 void launch_force(DeviceState& d, const SimConst& c, cudaStream_t s) {
     if (!d.n) return;
-    if (d.n < kForceTeamScene && !d.shared && standard_passes(d)) {
+    if (team_force(d)) {
         force_team_as<kIntegrate, kForceTeam, kForceTurn>(d, c, s);
         return;
     }
@@ -172,6 +174,13 @@ void launch_force(DeviceState& d, const SimConst& c, cudaStream_t s) {
 }  // namespace
 
 SF_INDEX_CHECK_ACCESSOR(index_check_failures_force)
+
+const char* force_kernel(const DeviceState& d) {
+    if (team_force(d)) return "force_team";
+    const bool lists = d.nbr && d.tune.list_mode != SF_LIST_NONE;
+    if (lists && d.tune.prefetch == 4) return d.tune.force_block == 256 ? "force_256_gather4" : "force_128_gather4";
+    return d.tune.force_block == 256 ? "force_256" : "force_128";
+}
 
 void launch_force_integrate(DeviceState& d, const SimConst& c, cudaStream_t s) { launch_force<true>(d, c, s); }
 

@@ -633,6 +633,17 @@ void enqueue_stage(uint32_t stage, DeviceState& d, const SimConst& c, cudaStream
     }
 }
 
+const char* stage_kernel(uint32_t stage, const DeviceState& d) {
+    if (!d.n || stage >= kNumStages) return "";
+    switch (stage) {
+        case 0: return density_kernel(d);
+        case 1: return force_kernel(d);
+        case 2: return "scan";
+        case 3: return d.cell_head ? "" : "scatter";
+        default: return d.cell_head ? "list_gather" : "rank_gather";
+    }
+}
+
 void enqueue_step(DeviceState& d, const SimConst& c, cudaStream_t s) {
     if (d.table && d.tune.batch_cluster && d.scene_order && d.scene_queue && d.n) {
         const int block = d.tune.batch_block ? d.tune.batch_block : 256;

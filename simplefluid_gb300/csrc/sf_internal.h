@@ -180,10 +180,9 @@ void launch_rank_gather(const DeviceState& d, cudaStream_t s);
 // eight, and its list would be walked entry by entry; there the indices are
 // bucketed (k_scatter) and read side by side.
 constexpr int kListedReach = 2;
-// Larger grids keep the bucketing too.  There the launch counts for little
+// Larger grids keep the bucketing too: the launch counts for little there
 // (1,048,576 particles, 8 million cells: 224.3 us a sub-step with lists, 227.0
-// without), the heads would be 32 MB more to keep, and the benchmark's contract
-// (tests/test_bench_contract.py) holds that scene to five launches.
+// without) and the heads would be 32 MB more to keep.
 constexpr uint32_t kListedCells = 4u << 20;
 // Scenes of fewer particles take the team forms (sf_team.cuh) of the two
 // passes.  Stage times in us, one thread per particle against the team
@@ -206,6 +205,8 @@ constexpr uint32_t kSmallBlockFrom = 81920, kSmallBlockTo = 262144;
 constexpr int kForceTeam = 2, kForceTurn = 4;
 // Whether the step uses the default kernel choices on a single scene.
 bool standard_passes(const DeviceState& d);
+const char* density_kernel(const DeviceState& d);
+const char* force_kernel(const DeviceState& d);
 void launch_density(const DeviceState& d, const SimConst& c, cudaStream_t s);
 // forces + symplectic Euler + box + next-step cell hash into pos2/vel2
 void launch_force_integrate(DeviceState& d, const SimConst& c, cudaStream_t s);
@@ -238,6 +239,8 @@ void enqueue_step(DeviceState& d, const SimConst& c, cudaStream_t s);
 constexpr uint32_t kNumStages = 5;
 extern const char* const kStageNames[kNumStages];
 void enqueue_stage(uint32_t stage, DeviceState& d, const SimConst& c, cudaStream_t s);
+// The kernel that the stage launches for this state ("" for none).
+const char* stage_kernel(uint32_t stage, const DeviceState& d);
 
 // ---- sub-step control (sf_frame.cu) ------------------------------------
 // Maxima of the uploaded state: |v|^2 over the particles, |a|^2 = 0.

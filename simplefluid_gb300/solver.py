@@ -243,6 +243,12 @@ class SPHSolver:
         C.check(self._lib.sf_get_tuning(self._ctx, byref(t)))
         return t
 
+    def stageKernels(self) -> dict:
+        """The kernel that each stage of a sub-step launches for the current
+        state and choices ("" for none)."""
+        return {self._lib.sf_stage_name(k).decode(): self._lib.sf_stage_kernel(self._ctx, k).decode()
+                for k in range(self._lib.sf_stage_count())}
+
     def deviceState(self) -> "C.sf_device_view":
         """Device pointers to the cell-sorted working arrays (sf_device_view)."""
         v = C.sf_device_view()
