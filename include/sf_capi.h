@@ -268,7 +268,12 @@ SF_API sf_status sf_test_fail_allocation(int64_t after);
 
 /* ---- kernel tuning -----------------------------------------------------------
  * Implementation choices of a context's step.  Every choice computes the same
- * bits; they differ only in speed.  Not part of the reference interface. */
+ * bits; they differ only in speed.  Not part of the reference interface.
+ * Until sf_set_tuning is called, the library chooses by the size of the scene:
+ * sf_get_tuning then reports the large scenes' blocks, and smaller scenes may
+ * take other blocks or several threads per particle (sf_stage_kernel says
+ * which).  From sf_set_tuning on the given blocks and gathers are used at every
+ * size, also where they equal the defaults. */
 #define SF_LIST_NONE 0        /* force pass rescans the candidate cells       */
 #define SF_LIST_TILE_STAGED 1 /* density pass stages neighbour lists in shared
                                  memory, writes 128-particle tiles             */

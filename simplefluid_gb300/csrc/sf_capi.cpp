@@ -511,7 +511,7 @@ sf_status copy_in(sf_ctx* ctx, void* dst, const void* src, size_t bytes) {
 constexpr uint32_t kSmallScene = 262144;
 
 void apply_size_defaults(sf_ctx* ctx) {
-    if (ctx->tune_explicit || ctx->d.table) return;  // batches use prefetch 2
+    if (ctx->d.tune.chosen || ctx->d.table) return;  // batches use prefetch 2
     const int pf = ctx->d.n < kSmallScene ? 4 : 2;
     if (ctx->d.tune.prefetch != pf) {
         ctx->d.tune.prefetch = pf;

@@ -66,7 +66,6 @@ struct sf_ctx {
     // tables (Grace: NVLink-C2C with address translation): -1 unknown, 0, 1
     int host_direct = -1;
     uint32_t* d_report = nullptr;  // sf_check_state counters
-    bool tune_explicit = false;    // sf_set_tuning was called: keep its choices
     cudaGraphExec_t step_graph = nullptr;  // one sub-step
     cudaGraphExec_t run_graph = nullptr;   // kRunSteps sub-steps
     cudaGraphExec_t call_graph = nullptr;  // call_steps sub-steps

@@ -235,7 +235,7 @@ SF_API sf_status sf_set_tuning(sf_ctx* ctx, const sf_tuning* t) {
     ctx->d.tune.l2_window = t->l2_window;
     ctx->d.tune.batch_cluster = t->batch_cluster;
     ctx->d.tune.batch_block = t->batch_block;
-    ctx->tune_explicit = true;
+    ctx->d.tune.chosen = true;
     drop_graph(ctx);
     return SF_OK;
 }

@@ -112,17 +112,12 @@ void density_as(const DeviceState& d, const SimConst& c, cudaStream_t s) {
 
 SF_INDEX_CHECK_ACCESSOR(index_check_failures_density)
 
-bool standard_passes(const DeviceState& d) {
-    const Tuning standard;
-    return !d.table && d.nbr && d.tune.list_mode == standard.list_mode &&
-           d.tune.density_block == standard.density_block && d.tune.force_block == standard.force_block &&
-           !d.tune.l2_window;
-}
+bool passes_by_size(const DeviceState& d) { return !d.table && d.nbr && !d.tune.chosen; }
 
 // The density pass's form: threads per block, or 0 for the team.
 static int density_form(const DeviceState& d) {
-    if (d.n < kDensityTeamScene && !d.shared && standard_passes(d)) return 0;
-    if (d.n >= kSmallBlockFrom && d.n < kSmallBlockTo && standard_passes(d)) return 128;
+    if (d.n < kDensityTeamScene && !d.shared && passes_by_size(d)) return 0;
+    if (d.n >= kSmallBlockFrom && d.n < kSmallBlockTo && passes_by_size(d)) return 128;
     if (d.nbr && d.tune.list_mode == SF_LIST_TILE_STAGED) return kNbTile;
     return d.tune.density_block;
 }

@@ -147,7 +147,7 @@ void force_as(DeviceState& d, const SimConst& c, cudaStream_t s) {
     });
 }
 
-bool team_force(const DeviceState& d) { return d.n < kForceTeamScene && !d.shared && standard_passes(d); }
+bool team_force(const DeviceState& d) { return d.n < kForceTeamScene && !d.shared && passes_by_size(d); }
 
 template <bool kIntegrate>
 void launch_force(DeviceState& d, const SimConst& c, cudaStream_t s) {

@@ -77,6 +77,7 @@ constexpr uint32_t kNear16 = 32767;
 
 // Kernel choices of a context (all give bit-identical results).
 struct Tuning {
+    bool chosen = false;           // by sf_set_tuning: taken as they are at every size
     int list_mode = SF_LIST_TILE;  // SF_LIST_*: how the density pass records neighbours
     int density_block = 256;       // 128 or 256 threads
     int force_block = 128;         // 128 or 256 threads
@@ -203,8 +204,9 @@ constexpr uint32_t kSmallBlockFrom = 81920, kSmallBlockTo = 262144;
 // (2 x 4; stage times at 16,000 and 32,000 particles 9.5 and 12.3 us, 4 x 4
 // 9.6 and 13.7, 3 x 2 9.6 and 13.9, 8 x 2 12.4 and 15.6).
 constexpr int kForceTeam = 2, kForceTurn = 4;
-// Whether the step uses the default kernel choices on a single scene.
-bool standard_passes(const DeviceState& d);
+// Whether the passes' forms go by the size of the scene: a single scene with lists
+// whose kernels the caller did not choose.
+bool passes_by_size(const DeviceState& d);
 const char* density_kernel(const DeviceState& d);
 const char* force_kernel(const DeviceState& d);
 void launch_density(const DeviceState& d, const SimConst& c, cudaStream_t s);

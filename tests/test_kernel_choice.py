@@ -3,7 +3,8 @@ import pytest
 
 from helpers import params_16k
 from simplefluid_gb300 import SPHSolver
-from test_contexts import cloud
+from simplefluid_gb300 import _capi as C
+from test_contexts import cloud, same_bits
 
 pytestmark = pytest.mark.gpu
 
@@ -24,3 +25,20 @@ def test_stages_report_their_kernels():
     with SPHSolver(params_16k(cellsPerH=1)) as s:
         s.setParticles(cloud(2000, 1))
         assert kernels(s)[2:] == ("scan", "scatter", "rank_gather")
+
+
+@pytest.mark.parametrize("n", [2000, 40000, 100000, 300000])
+def test_an_explicit_choice_is_taken_at_every_size(n):
+    """Also the blocks that sf_get_tuning reports before any choice; the state is the same."""
+    prm = params_16k(particleRadius=0.0025, kernelRadius=0.01)
+    pos = cloud(n, n, 0.3)
+    with SPHSolver(prm) as s:
+        s.setParticles(pos)
+        s.step(2)
+        want = s.getState()
+        for density, force, gather in ((256, 128, 2), (256, 128, 4), (128, 256, 4), (256, 256, 2)):
+            s.setTuning(C.sf_tuning(C.SF_LIST_TILE, density, force, gather))
+            s.setParticles(pos)
+            assert kernels(s)[:2] == (f"density_{density}", f"force_{force}" + ("_gather4" if gather == 4 else ""))
+            s.step(2)
+            same_bits(s.getState(), want)
