@@ -1056,6 +1056,8 @@ static sf_status add_frame_loop(sf_ctx* ctx, cudaGraph_t g, std::vector<cudaGrap
 // runs of sub-steps (of the lengths a frame has room for), then single ones up
 // to the frame's end.
 static sf_status build_frame_graph(sf_ctx* ctx, double frame_time, uint32_t max_substeps, cudaGraphExec_t* out) {
+    // the gather records' persisting-L2 window (reserved outside the captures)
+    if (ctx->d.tune.l2_window) sf::reserve_persisting_l2((size_t)ctx->d.n * 2 * sizeof(float4));
     cudaGraph_t g = nullptr;
     SF_CUDA(cudaGraphCreate(&g, 0));
     struct GraphGuard {

@@ -1,4 +1,8 @@
 """Which kernels a sub-step launches: by the size of the scene, unless the caller chose them."""
+import os
+import subprocess
+import sys
+
 import pytest
 
 from helpers import params_16k
@@ -42,3 +46,30 @@ def test_an_explicit_choice_is_taken_at_every_size(n):
             assert kernels(s)[:2] == (f"density_{density}", f"force_{force}" + ("_gather4" if gather == 4 else ""))
             s.step(2)
             same_bits(s.getState(), want)
+
+
+def test_frames_reserve_the_l2_window():
+    """A program that only runs frames gets the window it asked for (in a process of its own: the reservation is the
+    process's)."""
+    code = """
+import ctypes
+import numpy as np
+from simplefluid_gb300 import SPHParameters, SPHSolver
+from simplefluid_gb300 import _capi as C
+
+def reserved():
+    size = ctypes.c_size_t()
+    assert ctypes.CDLL("libcuda.so.1").cuCtxGetLimit(ctypes.byref(size), 6) == 0  # persisting L2
+    return size.value
+
+s = SPHSolver(SPHParameters(particleRadius=0.0025, kernelRadius=0.01))
+s.setTuning(C.sf_tuning(C.SF_LIST_TILE, 256, 128, 2, 1))
+s.setParticles(np.random.default_rng(1).random((1500000, 3)).astype(np.float32))
+assert reserved() < 1500000 * 32  # the device's default
+s.advanceFrames(1, 2e-4, 10)
+assert reserved() >= 1500000 * 32, reserved()
+s.close()
+"""
+    out = subprocess.run([sys.executable, "-c", code], capture_output=True, text=True, timeout=120,
+                         cwd=os.path.dirname(os.path.dirname(os.path.abspath(__file__))))
+    assert out.returncode == 0, out.stderr[-2000:]
