@@ -238,16 +238,19 @@ void drop_graph(sf_ctx* ctx) {
     ++ctx->gen;
 }
 
+// Whether the sort finds a cell's particles through lists.
+static bool wants_lists(const sf::SimConst& c) { return c.reach >= sf::kListedReach && c.ncells <= sf::kListedCells; }
+
 // On any failure the grid is released and the context needs a new upload.
 sf_status alloc_grid(sf_ctx* ctx) {
     sf::DeviceState& d = ctx->d;
-    if (d.ncells == ctx->c.ncells && d.counts) return SF_OK;
+    const bool lists = wants_lists(ctx->c);
+    if (d.ncells == ctx->c.ncells && d.counts && (d.cell_head != nullptr) == lists) return SF_OK;
     free_grid(d);
     const uint64_t pad = ((uint64_t)ctx->c.ncells + 1 + sf::kScanTile - 1) / sf::kScanTile * sf::kScanTile;
     const uint32_t ntiles = (uint32_t)(pad / sf::kScanTile);
     // one allocation: the histogram, the cell table, the scan-tile totals and,
     // where cells have lists, their heads
-    const bool lists = ctx->c.reach >= sf::kListedReach && ctx->c.ncells <= sf::kListedCells;
     const size_t words = 2 * pad + ntiles + (lists ? pad : 0);
     cudaError_t e = dev_malloc(&d.counts, words * sizeof(uint32_t));
     if (e == cudaSuccess) e = cudaMemsetAsync(d.counts, 0, (2 * pad + ntiles) * sizeof(uint32_t), ctx->stream);
@@ -815,7 +818,8 @@ SF_API sf_status sf_set_params(sf_ctx* ctx, const sf_params* p) {
     SF_TRY(wait_stream(ctx));
     const bool grid_changed = std::memcmp(c.n, ctx->c.n, sizeof(c.n)) != 0 ||
                               std::memcmp(c.bmin, ctx->c.bmin, sizeof(c.bmin)) != 0 ||
-                              std::memcmp(c.inv_cell, ctx->c.inv_cell, sizeof(c.inv_cell)) != 0;
+                              std::memcmp(c.inv_cell, ctx->c.inv_cell, sizeof(c.inv_cell)) != 0 ||
+                              wants_lists(c) != wants_lists(ctx->c);
     const bool became_adaptive = c.adaptive && !ctx->c.adaptive;
     ctx->params = *p;
     ctx->c = c;

@@ -73,3 +73,23 @@ s.close()
     out = subprocess.run([sys.executable, "-c", code], capture_output=True, text=True, timeout=120,
                          cwd=os.path.dirname(os.path.dirname(os.path.abspath(__file__))))
     assert out.returncode == 0, out.stderr[-2000:]
+
+
+def test_the_sort_follows_the_grid_not_its_history():
+    """The same cells as one per h and as two per 2h: the kernels and the state of a context that switches, with and
+    without particles, are those of a new one."""
+    both = [params_16k(kernelRadius=h, cellsPerH=k) for h, k in ((0.04, 1), (0.08, 2))]
+    pos = cloud(3000, 3)
+    with SPHSolver(both[1]) as s:
+        for prm, other in (both, both[::-1], both):
+            s.setParams(prm)
+            s.setParticles(pos)
+            s.setParams(other)
+            s.setParams(prm)
+            with SPHSolver(prm) as new:
+                new.setParticles(pos)
+                assert s.gridDims() == new.gridDims()
+                assert kernels(s) == kernels(new)
+                s.step(3)
+                new.step(3)
+                same_bits(s.getState(), new.getState())
