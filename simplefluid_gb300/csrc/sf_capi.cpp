@@ -648,6 +648,7 @@ int derive_constants(const sf_params& p, SimConst* c, const char** why) {
     c->cfl_a = 0.25f;
     const int K = p.cells_per_h ? p.cells_per_h : 2;
     c->reach = K;
+    c->lists_fit = 4.0 / 3.0 * kPi * std::pow(h / (2.0 * r), 3) <= kNbCap ? 1 : 0;
     double coord_max = 0.0;
     uint64_t cells = 1;
     for (int a = 0; a < 3; ++a) {

@@ -245,7 +245,7 @@ SF_API uint32_t sf_stage_count(void) { return sf::kNumStages; }
 SF_API const char* sf_stage_name(uint32_t stage) { return stage < sf::kNumStages ? sf::kStageNames[stage] : ""; }
 
 SF_API const char* sf_stage_kernel(const sf_ctx* ctx, uint32_t stage) {
-    return ctx ? sf::stage_kernel(stage, ctx->d) : "";
+    return ctx ? sf::stage_kernel(stage, ctx->d, ctx->c) : "";
 }
 
 SF_API sf_status sf_profile_steps(sf_ctx* ctx, uint32_t nsteps, uint64_t flush_bytes, float* stage_ms,

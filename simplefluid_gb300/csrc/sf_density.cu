@@ -79,7 +79,10 @@ __global__ void __launch_bounds__((2 * kReach + 1) * 32)
                    FrameState* __restrict__ frame) {
     __shared__ DensityTeamShared<kReach> sh;
     grid_dependency_wait();
-    allow_dependents_sized(n);
+    // The next launch is released when the blocks end: the force pass's blocks,
+    // launched early, crowd as in mid-size scenes.  A sub-step in disorder, early /
+    // late: 18,000 particles 19.6 / 17.9 us (with one cell per h 27.2 / 25.9, three
+    // 22.2 / 19.7), 30,000 24.2 / 22.4, 8,000 15.5 / 15.5, 1,331 13.5 / 14.0.
     if (frame && blockIdx.x == 0 && threadIdx.x == 0) choose_dt(frame, c);
     const uint32_t i = blockIdx.x * kTeamParticles + (threadIdx.x & 31u);
     density_team<kReach>(min(i, n - 1), i < n, c, pos, cs, n, rho_out, pr_out, nbr, nbr_count, vel, pv, sh);
@@ -115,21 +118,21 @@ SF_INDEX_CHECK_ACCESSOR(index_check_failures_density)
 bool passes_by_size(const DeviceState& d) { return !d.table && d.nbr && !d.tune.chosen; }
 
 // The density pass's form: threads per block, or 0 for the team.
-static int density_form(const DeviceState& d) {
-    if (d.n < kDensityTeamScene && !d.shared && passes_by_size(d)) return 0;
+static int density_form(const DeviceState& d, const SimConst& c) {
+    if (team_scene(d, c, kDensityTeamScene)) return 0;
     if (d.n >= kSmallBlockFrom && d.n < kSmallBlockTo && passes_by_size(d)) return 128;
     if (d.nbr && d.tune.list_mode == SF_LIST_TILE_STAGED) return kNbTile;
     return d.tune.density_block;
 }
 
-const char* density_kernel(const DeviceState& d) {
-    const int form = density_form(d);
+const char* density_kernel(const DeviceState& d, const SimConst& c) {
+    const int form = density_form(d, c);
     return form == 0 ? "density_team" : form == 128 ? "density_128" : "density_256";
 }
 
 void launch_density(const DeviceState& d, const SimConst& c, cudaStream_t s) {
     if (!d.n) return;
-    const int form = density_form(d);
+    const int form = density_form(d, c);
     if (form == 0) {
         with_reach(c.reach, [&](auto R) {
             constexpr int K = decltype(R)::value;

@@ -40,13 +40,13 @@ inline int sm_count() {
 __device__ __forceinline__ void grid_dependency_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void allow_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
-// The same in the passes of mid-size scenes only when a block ends.  Their
-// grids are about one wave: the next kernel's blocks, launched early, go where
-// the running blocks leave room, and the SMs they crowd on finish last.  Larger
-// scenes gain from blocks that are in place when the last wave ends, smaller
-// ones (teams) leave room everywhere.  Ten sub-steps in disorder, early / late:
-// 40,000 particles 333 / 316 us, 90,000 468 / 432, 150,000 637 / 623, 200,000
-// 757 / 753 (and 236,987 918 / 931); 16,000 152 / 154.
+// The same in the one-thread passes of mid-size scenes only when a block ends.
+// Their grids are about one wave: the next kernel's blocks, launched early, go
+// where the running blocks leave room, and the SMs they crowd on finish last.
+// Larger scenes gain from blocks that are in place when the last wave ends, smaller
+// ones leave room everywhere.  Ten sub-steps in disorder, early / late: 40,000
+// particles 333 / 316 us, 90,000 468 / 432, 150,000 637 / 623, 200,000 757 / 753
+// (and 236,987 918 / 931).
 __device__ __forceinline__ void allow_dependents_sized(uint32_t n) {
     if (n < kForceTeamScene || n >= kEarlyLaunchScene) allow_dependents();
 }

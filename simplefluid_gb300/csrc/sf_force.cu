@@ -147,12 +147,12 @@ void force_as(DeviceState& d, const SimConst& c, cudaStream_t s) {
     });
 }
 
-bool team_force(const DeviceState& d) { return d.n < kForceTeamScene && !d.shared && passes_by_size(d); }
+bool team_force(const DeviceState& d, const SimConst& c) { return team_scene(d, c, kForceTeamScene); }
 
 template <bool kIntegrate>
 void launch_force(DeviceState& d, const SimConst& c, cudaStream_t s) {
     if (!d.n) return;
-    if (team_force(d)) {
+    if (team_force(d, c)) {
         force_team_as<kIntegrate, kForceTeam, kForceTurn>(d, c, s);
         return;
     }
@@ -175,8 +175,8 @@ void launch_force(DeviceState& d, const SimConst& c, cudaStream_t s) {
 
 SF_INDEX_CHECK_ACCESSOR(index_check_failures_force)
 
-const char* force_kernel(const DeviceState& d) {
-    if (team_force(d)) return "force_team";
+const char* force_kernel(const DeviceState& d, const SimConst& c) {
+    if (team_force(d, c)) return "force_team";
     const bool lists = d.nbr && d.tune.list_mode != SF_LIST_NONE;
     if (lists && d.tune.prefetch == 4) return d.tune.force_block == 256 ? "force_256_gather4" : "force_128_gather4";
     return d.tune.force_block == 256 ? "force_256" : "force_128";

@@ -633,11 +633,11 @@ void enqueue_stage(uint32_t stage, DeviceState& d, const SimConst& c, cudaStream
     }
 }
 
-const char* stage_kernel(uint32_t stage, const DeviceState& d) {
+const char* stage_kernel(uint32_t stage, const DeviceState& d, const SimConst& c) {
     if (!d.n || stage >= kNumStages) return "";
     switch (stage) {
-        case 0: return density_kernel(d);
-        case 1: return force_kernel(d);
+        case 0: return density_kernel(d, c);
+        case 1: return force_kernel(d, c);
         case 2: return "scan";
         case 3: return d.cell_head ? "" : "scatter";
         default: return d.cell_head ? "list_gather" : "rank_gather";

@@ -36,6 +36,7 @@ struct SimConst {
     // adaptive sub-step: dt = min(dt_max, cfl_v h / max|v|, cfl_a sqrt(h / max|a|))
     int adaptive;
     float cfl_v, cfl_a;
+    int lists_fit;        // at rest (particles 2r apart) a neighbour list holds all within h
 };
 
 // Device-side frame and sub-step state (one per context).
@@ -186,11 +187,18 @@ constexpr int kListedReach = 2;
 // without) and the heads would be 32 MB more to keep.
 constexpr uint32_t kListedCells = 4u << 20;
 // Scenes of fewer particles take the team forms (sf_team.cuh) of the two
-// passes.  Stage times in us, one thread per particle against the team
-// (jittered lattice; disordered): density 16.4 / 10.3 at 16,000 particles,
-// 23.8 / 20.0; 25.1 / 23.9 at 56,000, 24.5 / 24.6 at 65,536 (disordered);
-// force 12.3 / 9.5 at 16,000, 12.9 / 12.3; 14.7 / 14.3 at 32,000, 13.1 / 16.1
-// at 48,000.
+// passes.  Stage times in us, one thread per particle / the team (jittered
+// lattice; disordered), two cells per h: density 18.4 / 10.3; 22.4 / 12.4 at 16,000
+// particles, 20.2 / 17.2; 24.4 / 22.6 at 50,000, 24.5 / 20.3; 24.6 / 23.6 at 56,000.
+// One cell per h: 24.4 / 14.4; 26.4 / 16.3 at 16,000, 28.4 / 24.4; 31.9 / 27.0 at
+// 56,000.  Three: 22.3 / 12.5; 31.0 / 14.2 and 24.6 / 26.9; 34.9 / 31.2.  Force
+// 12.3 / 8.5; 14.4 / 10.1 at 16,000, 12.4 / 10.1; 14.5 / 10.9 at 30,000, 12.5 /
+// 13.1; 14.4 / 14.7 at 40,000.
+// Where a list cannot hold the neighbours at rest (h above 4.9 particle radii)
+// both passes walk the candidates anyway and a team only takes room: a sub-step
+// of 16,000 to 30,000 particles at 6 radii was 0.72 to 1.0 of one thread's speed.
+// Scenes compressed that far with h = 4.5 radii: 0.98 to 1.14 with two or three
+// cells per h, about 0.9 with one.
 constexpr uint32_t kDensityTeamScene = 57344, kForceTeamScene = 32768;
 // Scenes from this size on launch the next pass early (allow_dependents_sized).
 constexpr uint32_t kEarlyLaunchScene = 196608;
@@ -207,8 +215,12 @@ constexpr int kForceTeam = 2, kForceTurn = 4;
 // Whether the passes' forms go by the size of the scene: a single scene with lists
 // whose kernels the caller did not choose.
 bool passes_by_size(const DeviceState& d);
-const char* density_kernel(const DeviceState& d);
-const char* force_kernel(const DeviceState& d);
+// Whether a pass takes its team form below `limit` particles.
+inline bool team_scene(const DeviceState& d, const SimConst& c, uint32_t limit) {
+    return d.n < limit && !d.shared && c.lists_fit && passes_by_size(d);
+}
+const char* density_kernel(const DeviceState& d, const SimConst& c);
+const char* force_kernel(const DeviceState& d, const SimConst& c);
 void launch_density(const DeviceState& d, const SimConst& c, cudaStream_t s);
 // forces + symplectic Euler + box + next-step cell hash into pos2/vel2
 void launch_force_integrate(DeviceState& d, const SimConst& c, cudaStream_t s);
@@ -242,7 +254,7 @@ constexpr uint32_t kNumStages = 5;
 extern const char* const kStageNames[kNumStages];
 void enqueue_stage(uint32_t stage, DeviceState& d, const SimConst& c, cudaStream_t s);
 // The kernel that the stage launches for this state ("" for none).
-const char* stage_kernel(uint32_t stage, const DeviceState& d);
+const char* stage_kernel(uint32_t stage, const DeviceState& d, const SimConst& c);
 
 // ---- sub-step control (sf_frame.cu) ------------------------------------
 // Maxima of the uploaded state: |v|^2 over the particles, |a|^2 = 0.

@@ -44,11 +44,12 @@ struct DensityTeamShared {
     float q[kNbCap][kTeamParticles];                       // h^2 - r^2 of the particles' neighbours, in order
     uint32_t count[2 * kReach + 1][kTeamParticles];        // neighbours found in each plane
 };
-constexpr uint32_t kPlaneOverflow = 1u << 16;  // a plane's count where a row holds more than 32 candidates
+constexpr uint32_t kPlaneOverflow = 1u << 16;  // a plane's count where a row holds more candidates than its mask
 
 // Density of the block's particles (particle i of this lane; live: i < n).  A
 // thread keeps a bit per candidate of its plane; once the team's counts are
-// known it writes its neighbours to their places.
+// known it writes its neighbours to their places, kNbCap places at a time: more
+// than a list holds are summed in further rounds.
 template <int kReach>
 __device__ __forceinline__ void density_team(uint32_t i, bool live, const SimConst& c, const float4* __restrict__ pos,
                                              const uint32_t* __restrict__ cs, uint32_t n, float* __restrict__ rho_out,
@@ -56,6 +57,10 @@ __device__ __forceinline__ void density_team(uint32_t i, bool live, const SimCon
                                              uint32_t* __restrict__ nbr_count, const float4* __restrict__ vel,
                                              float4* __restrict__ pv, DensityTeamShared<kReach>& sh) {
     constexpr int kTeam = 2 * kReach + 1;
+    // Words of a row's mask.  At rest a row of one cell per h (2r = h / 2) holds 24
+    // candidates and in compressed places more than 64; with two or three per
+    // h it holds 5 or 2.
+    constexpr int kWords = kReach == 1 ? 3 : 1;
     const int lane = (int)(threadIdx.x & 31u), part = (int)(threadIdx.x / 32u);
     const float4 xi = ldg4(pos + i);
     const CellPoint p = cell_point(c, xi.x, xi.y, xi.z);
@@ -100,36 +105,39 @@ __device__ __forceinline__ void density_team(uint32_t i, bool live, const SimCon
     // flight together.  r^2 - h^2 is negative where a candidate is a
     // neighbour: its sign bit is shifted into the row's mask.  Past its row's
     // end a thread tests the particle itself, moved out of reach.
-    uint32_t near[kTeam], mine = 0, most = 0;
+    uint32_t near[kTeam][kWords], past[kWords], mine = 0, most = 0;  // past: one past the candidates in a word
 #pragma unroll
-    for (int q = 0; q < kTeam; ++q) {
-        near[q] = 0u;
-        most = max(most, len[q]);
-    }
-    uint32_t tested = 0;
+    for (int q = 0; q < kTeam; ++q) most = max(most, len[q]);
+#pragma unroll
+    for (int w = 0; w < kWords; ++w) {
+#pragma unroll
+        for (int q = 0; q < kTeam; ++q) near[q][w] = 0u;
+        uint32_t tested = 32u * w;
 #pragma unroll 1
-    for (; tested < min(most, 32u); tested += 2) {
-        float4 x0[kTeam], x1[kTeam];
+        for (; tested < min(most, 32u * w + 32u); tested += 2) {
+            float4 x0[kTeam], x1[kTeam];
 #pragma unroll
-        for (int q = 0; q < kTeam; ++q) {
-            const uint32_t j = end[q] - len[q] + tested;
-            x0[q] = ldg4(pos + (tested < len[q] ? j : i));
-            x1[q] = ldg4(pos + (tested + 1 < len[q] ? j + 1 : i));
-        }
+            for (int q = 0; q < kTeam; ++q) {
+                const uint32_t j = end[q] - len[q] + tested;
+                x0[q] = ldg4(pos + (tested < len[q] ? j : i));
+                x1[q] = ldg4(pos + (tested + 1 < len[q] ? j + 1 : i));
+            }
 #pragma unroll
-        for (int q = 0; q < kTeam; ++q) {
-            if (!(tested < len[q])) x0[q].x = __int_as_float(0x7f800000);
-            if (!(tested + 1 < len[q])) x1[q].x = __int_as_float(0x7f800000);
-            const F2 dx = f2(xi.x - x0[q].x, xi.x - x1[q].x), dy = f2(xi.y - x0[q].y, xi.y - x1[q].y),
-                     dz = f2(xi.z - x0[q].z, xi.z - x1[q].z);
-            const float2 u = unpack(add2(fma2(dz, dz, fma2(dy, dy, mul2(dx, dx))), f2(-c.h2, -c.h2)));
-            near[q] = __funnelshift_l(__float_as_uint(u.x), near[q], 1);
-            near[q] = __funnelshift_l(__float_as_uint(u.y), near[q], 1);
+            for (int q = 0; q < kTeam; ++q) {
+                if (!(tested < len[q])) x0[q].x = __int_as_float(0x7f800000);
+                if (!(tested + 1 < len[q])) x1[q].x = __int_as_float(0x7f800000);
+                const F2 dx = f2(xi.x - x0[q].x, xi.x - x1[q].x), dy = f2(xi.y - x0[q].y, xi.y - x1[q].y),
+                         dz = f2(xi.z - x0[q].z, xi.z - x1[q].z);
+                const float2 u = unpack(add2(fma2(dz, dz, fma2(dy, dy, mul2(dx, dx))), f2(-c.h2, -c.h2)));
+                near[q][w] = __funnelshift_l(__float_as_uint(u.x), near[q][w], 1);
+                near[q][w] = __funnelshift_l(__float_as_uint(u.y), near[q][w], 1);
+            }
         }
+        past[w] = tested;
+#pragma unroll
+        for (int q = 0; q < kTeam; ++q) mine += (uint32_t)__popc(near[q][w]);
     }
-#pragma unroll
-    for (int q = 0; q < kTeam; ++q) mine += (uint32_t)__popc(near[q]);
-    sh.count[part][lane] = most > 32u ? kPlaneOverflow : mine;
+    sh.count[part][lane] = most > 32u * kWords ? kPlaneOverflow : mine;
     __syncthreads();
     uint32_t at = 0, cnt = 0;
 #pragma unroll
@@ -138,38 +146,65 @@ __device__ __forceinline__ void density_team(uint32_t i, bool live, const SimCon
         at += k < part ? v : 0u;
         cnt += v;
     }
-    const bool fits = cnt <= (uint32_t)kNbCap;
-    if (fits) {
-        uint32_t* const lst = nbr + nbr_index(i, 0);
+    const bool masked = cnt < kPlaneOverflow, list = live && cnt <= (uint32_t)kNbCap;
+    const uint32_t most_near = __reduce_max_sync(0xffffffffu, masked ? cnt : 0u);  // the same in every warp
+    uint32_t* const lst = nbr + nbr_index(i, 0);
+    // the thread's neighbours from where it stopped up to place `to`; place `base` is the first of this round
+    auto write = [&](uint32_t base, auto bounded, uint32_t to) {
 #pragma unroll
         for (int q = 0; q < kTeam; ++q) {
+#pragma unroll
+            for (int w = 0; w < kWords; ++w) {
+                uint32_t m = near[q][w];
 #pragma unroll 1
-            for (uint32_t m = near[q]; m; ++at) {
-                const uint32_t b = 31u - (uint32_t)__clz((int)m), j = end[q] - len[q] + tested - 1u - b;
-                m ^= 1u << b;
-                sh.q[at][lane] = c.h2 - r2_of(ldg4(pos + j));
-                if (live) lst[(size_t)at * kNbTile] = j;
+                for (; m && (!decltype(bounded)::value || at < to); ++at) {
+                    const uint32_t b = 31u - (uint32_t)__clz((int)m), j = end[q] - len[q] + past[w] - 1u - b;
+                    m ^= 1u << b;
+                    sh.q[at - base][lane] = c.h2 - r2_of(ldg4(pos + j));
+                    if (list) lst[(size_t)at * kNbTile] = j;
+                }
+                if (decltype(bounded)::value) near[q][w] = m;
             }
         }
-        const uint32_t k = cnt + (uint32_t)part;
-        if (k < ((cnt + 3u) & ~3u)) sh.q[k][lane] = 0.f;  // zero terms, to a multiple of four
+    };
+    float s = 0.f;
+    auto sum = [&](uint32_t terms) {
+        for (uint32_t k = 0; k < terms; k += 4) {
+#pragma unroll
+            for (uint32_t u = 0; u < 4; ++u) {
+                const float q = sh.q[k + u][lane];
+                s = fmaf(q * q, q, s);
+            }
+        }
+    };
+    auto pad = [&](uint32_t terms) {  // zero terms, to a multiple of four
+        const uint32_t k = terms + (uint32_t)part;
+        if (k < ((terms + 3u) & ~3u)) sh.q[k][lane] = 0.f;
+    };
+    if (most_near <= (uint32_t)kNbCap) {
+        const uint32_t terms = masked ? cnt : 0u;
+        if (masked) write(0, std::false_type{}, 0);
+        pad(terms);
+        __syncthreads();
+        if (part == 0) sum(terms);
+    } else {
+#pragma unroll 1
+        for (uint32_t base = 0; base < most_near; base += kNbCap) {
+            const uint32_t terms = masked && cnt > base ? min(cnt - base, (uint32_t)kNbCap) : 0u;
+            if (terms) write(base, std::true_type{}, base + kNbCap);
+            pad(terms);
+            __syncthreads();
+            if (part == 0) sum(terms);
+            __syncthreads();
+        }
     }
-    __syncthreads();
     if (part != 0 || !live) return;
-    if (!fits) {  // a dense place: more neighbours than a list holds, or than 31 candidates in a row
+    if (!masked) {  // a very dense place
         density_one<kEmitTile, kReach>(i, c, xi, pos, cs, n, rho_out, pr_out, nbr, nbr_count, vel, pv, false, nullptr,
                                        0);
         return;
     }
     const float4 v = ldg4(vel + i);
-    float s = 0.f;
-    for (uint32_t k = 0; k < cnt; k += 4) {
-#pragma unroll
-        for (uint32_t u = 0; u < 4; ++u) {
-            const float q = sh.q[k + u][lane];
-            s = fmaf(q * q, q, s);
-        }
-    }
     const float rho = c.cd * s;
     const float pi = pressure_of(c, rho), inv_rho = 1.f / rho;
     rho_out[i] = rho;
@@ -187,10 +222,26 @@ struct ForceTeamShared {
     uint32_t small[kTeamParticles];  // PairSums::small so far
 };
 
-// Named barriers of two warps (ids from 1; 0 is __syncthreads): the warp that
-// hands on arrives, the next one waits.
-__device__ __forceinline__ void turn_wait(int warp) { asm volatile("bar.sync %0, 64;" ::"r"(1 + warp) : "memory"); }
-__device__ __forceinline__ void turn_pass(int warp) { asm volatile("bar.arrive %0, 64;" ::"r"(1 + warp) : "memory"); }
+// Named barriers of the two warps (1 + warp; 0 is __syncthreads): the warp that
+// hands on arrives, the next one waits.  Their numbers are constants: with a
+// number in a register a block holds all 16 barriers, and fewer blocks fit an SM
+// (force stage at 30,000 particles 12.8 -> 10.2 us, disordered 14.4 -> 11.4).
+template <int kTeam>
+__device__ __forceinline__ void turn_wait(int warp) {
+    static_assert(kTeam == 2, "one barrier per warp");
+    if (warp == 0)
+        asm volatile("bar.sync 1, 64;" ::: "memory");
+    else
+        asm volatile("bar.sync 2, 64;" ::: "memory");
+}
+template <int kTeam>
+__device__ __forceinline__ void turn_pass(int warp) {
+    static_assert(kTeam == 2, "one barrier per warp");
+    if (warp == 0)
+        asm volatile("bar.arrive 1, 64;" ::: "memory");
+    else
+        asm volatile("bar.arrive 2, 64;" ::: "memory");
+}
 
 // The force sums of particle i (of this lane), and false where the list
 // overflowed or a distance lies outside root_quotient's range.  They are those
@@ -260,7 +311,7 @@ __device__ __forceinline__ bool force_team(uint32_t i, const uint32_t* __restric
         gather();
         entries();
         if (t > 0) {
-            turn_wait(part);
+            turn_wait<kTeam>(part);
             const float2 ux = sh.sum[0][lane], uy = sh.sum[1][lane], uz = sh.sum[2][lane];
             small = min(small, sh.small[lane]);
             sx = f2(ux.x, ux.y), sy = f2(uy.x, uy.y), sz = f2(uz.x, uz.y);
@@ -276,7 +327,7 @@ __device__ __forceinline__ bool force_team(uint32_t i, const uint32_t* __restric
             sh.sum[1][lane] = unpack(sy);
             sh.sum[2][lane] = unpack(sz);
             sh.small[lane] = small;
-            turn_pass(next_part);
+            turn_pass<kTeam>(next_part);
         }
     }
     const float2 ux = unpack(sx), uy = unpack(sy), uz = unpack(sz);

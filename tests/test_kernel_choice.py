@@ -93,3 +93,11 @@ def test_the_sort_follows_the_grid_not_its_history():
                 s.step(3)
                 new.step(3)
                 same_bits(s.getState(), new.getState())
+
+
+@pytest.mark.parametrize("cells", [1, 2, 3])
+@pytest.mark.parametrize("ratio,team", [(4.0, True), (4.9, True), (5.0, False), (8.0, False)])
+def test_no_teams_where_the_lists_overflow_at_rest(ratio, team, cells):
+    with SPHSolver(params_16k(kernelRadius=0.01 * ratio, cellsPerH=cells)) as s:
+        s.setParticles(cloud(2000, 1))
+        assert kernels(s)[:2] == (("density_team", "force_team") if team else ("density_256", "force_128_gather4"))

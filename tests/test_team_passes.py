@@ -139,3 +139,14 @@ def test_sizes_where_the_blocks_and_launches_change(n):
         s.setTuning(t)
 
     same(run(prm, pos, vel), run(prm, pos, vel, blocks_256))
+
+
+@pytest.mark.parametrize("cells", [1, 2, 3])
+@pytest.mark.parametrize("spacing", [0.0165, 0.0145, 0.0125, 0.0105])
+def test_more_neighbours_than_a_list_holds(spacing, cells):
+    """Lattices of about 60, 88, 137 and 232 neighbours: lists that just overflow, sums in up to four rounds, rows of
+    more than 32, 64 and 96 candidates."""
+    pos, vel = block(3001, 9, spacing=spacing, jitter=0.2)
+    got = run(params_16k(cellsPerH=cells, timeStep=1e-6), pos, vel)
+    assert got[3] > 0
+    same(got, run(params_16k(cellsPerH=cells, timeStep=1e-6), pos, vel, one_thread))
