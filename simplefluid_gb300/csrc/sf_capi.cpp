@@ -319,7 +319,7 @@ sf_status check_launch(const char* what) {
 // Load a caller-order AoS state from device arrays (vel3 NULL: at rest) and
 // sort it into the cell order.
 sf_status sort_uploaded(sf_ctx* ctx, const float* pos3, const float* vel3) {
-    sf::DeviceState& d = ctx->d;
+    sf::DeviceState d = sf::upload_view(ctx->d);
     sf::launch_load_hash(d, pos3, vel3, d.vel2, ctx->c, ctx->stream);
     sf::enqueue_sort_tail(d, ctx->stream);
     if (ctx->frame && ctx->c.adaptive) sf::launch_init_maxima(d.vel, d.n, ctx->frame, ctx->stream);
@@ -341,7 +341,7 @@ sf_status need_aux(sf_ctx* ctx) {
 // scattered; the gather waits for the velocities.  ev_in marks the end of
 // both copies (the velocity copy starts after the position copy).
 sf_status upload_overlapped(sf_ctx* ctx, const float* pos_xyz, const float* vel_xyz) {
-    sf::DeviceState& d = ctx->d;
+    sf::DeviceState d = sf::upload_view(ctx->d);
     SF_TRY(need_aux(ctx));
     const size_t bytes = (size_t)d.n * 3 * sizeof(float);
     float* io_pos = d.io;
@@ -830,7 +830,7 @@ SF_API sf_status sf_set_params(sf_ctx* ctx, const sf_params* p) {
         SF_TRY(alloc_grid(ctx));
         if (ctx->sorted && ctx->d.n) {
             // Re-bucket the current state on the new grid (positions unchanged).
-            sf::DeviceState& d = ctx->d;
+            sf::DeviceState d = sf::upload_view(ctx->d);
             SF_CUDA(cudaMemcpyAsync(d.pos2, d.pos, (size_t)d.n * sizeof(float4), cudaMemcpyDeviceToDevice,
                                     ctx->stream));
             SF_CUDA(cudaMemcpyAsync(d.vel2, d.vel, (size_t)d.n * sizeof(float4), cudaMemcpyDeviceToDevice,

@@ -225,7 +225,7 @@ SF_API sf_status sf_batch_set_cells_per_h(sf_batch* b, int32_t cells_per_h) {
     drop_graph(&b->eng);
     SF_TRY(alloc_grid(&b->eng));
     SF_TRY(batch_upload_table(b));
-    sf::DeviceState& d = b->eng.d;
+    sf::DeviceState d = sf::upload_view(b->eng.d);
     if (b->eng.sorted && d.n) {
         // re-bucket the current state on the new grids (positions unchanged)
         SF_CUDA(cudaMemcpyAsync(d.pos2, d.pos, (size_t)d.n * sizeof(float4), cudaMemcpyDeviceToDevice, b->eng.stream));

@@ -495,7 +495,7 @@ SF_API sf_status sf_load_state(sf_ctx* ctx, const char* path, double* sim_time_o
     ctx->sorted = false;
     apply_size_defaults(ctx);
     if (n) {
-        sf::DeviceState& d = ctx->d;
+        sf::DeviceState d = sf::upload_view(ctx->d);
         SF_TRY(copy_in(ctx, d.io, pv.data(), pv.size() * sizeof(float)));
         SF_TRY(copy_in(ctx, d.tmp, ids.data(), ids.size() * sizeof(uint32_t)));
         sf::launch_load_sorted(d.io, d.io + 3 * (size_t)n, d.tmp, n, d.pos2, d.vel2, ctx->stream);

@@ -9,7 +9,8 @@
 // previous order) is restored by ranking each particle among its cell's
 // members, which makes the order deterministic and identical to a stable sort.
 // The members are found by the list that the histogram pass threads through
-// them or, in cells of the kernel radius's size, by bucketing their indices.
+// them or, in cells of the kernel radius's size, in large grids and in uploads, by
+// bucketing their indices.
 #include <mutex>
 
 #include "sf_device.cuh"

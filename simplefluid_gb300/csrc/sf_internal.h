@@ -178,14 +178,30 @@ void launch_scatter(const DeviceState& d, cudaStream_t s);
 void launch_rank_gather(const DeviceState& d, cudaStream_t s);
 // Cells of this many per kernel radius or more (at rest one particle a cell)
 // are sorted through lists, one launch less: a sub-step of 16,000 particles
-// 18.2 -> 16.7 us, of 236,987 95 -> 93.  A cell of the kernel radius itself holds
-// eight, and its list would be walked entry by entry; there the indices are
-// bucketed (k_scatter) and read side by side.
+// 18.2 -> 16.7 us, of 236,987 95 -> 93.  Cells of the kernel radius itself hold
+// eight and are bucketed (k_scatter): lists were neither faster nor slower there
+// (20 sub-steps of 16,000 particles 681 against 683 us).
 constexpr int kListedReach = 2;
 // Larger grids keep the bucketing too: the launch counts for little there
 // (1,048,576 particles, 8 million cells: 224.3 us a sub-step with lists, 227.0
 // without) and the heads would be 32 MB more to keep.
 constexpr uint32_t kListedCells = 4u << 20;
+// A list is walked entry by entry, so a crowded cell takes longer than bucketed
+// indices do: the sort of 200,000 particles in cells of 16 members 21 us against 25,
+// of 64 31 against 26, of 512 107 against 42.  The box keeps the particles of a
+// running scene from such crowds (64 members are 60 times the rest density, and
+// the passes then take 150 us and more), but an upload may place any number
+// outside it, all in a few cells of its border.  Uploads of this many particles or
+// more are therefore bucketed.  Upload and sort in us, list / bucketing, with
+// none, 1%, 10% and all particles outside: 65,536 particles 31 / 33, 154 / 51,
+// 1185 / 185, 6367 / 1526; 4,096 28 / 31, 36 / 32, 95 / 40, 358 / 127; 1,331 28 /
+// 31, 29 / 30, 48 / 33, 135 / 63, where the launch counts most and a crowd least.
+constexpr uint32_t kListedUpload = 2048;
+// The state as the sort of an upload takes it.
+inline DeviceState upload_view(DeviceState d) {
+    if (d.n >= kListedUpload) d.cell_head = nullptr;
+    return d;
+}
 // Scenes of fewer particles take the team forms (sf_team.cuh) of the two
 // passes.  Stage times in us, one thread per particle / the team (jittered
 // lattice; disordered), two cells per h: density 18.4 / 10.3; 22.4 / 12.4 at 16,000

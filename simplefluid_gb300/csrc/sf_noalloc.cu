@@ -157,8 +157,10 @@ int noalloc_density(const sf_params& p, const SimConst& c, const float* d_pos_xy
     d.pr = reinterpret_cast<float2*>(base + kOffPr);
     d.rho = reinterpret_cast<float*>(base + kOffRho);
     d.key_slot = reinterpret_cast<uint2*>(base + kOffKeySlot);
-    // the heads of the cells' lists, or the bucketed indices
-    (c.reach >= kListedReach ? d.cell_head : d.tmp) = reinterpret_cast<uint32_t*>(base + kOffTmp);
+    // the bucketed indices, or the heads of the cells' lists
+    d.tmp = reinterpret_cast<uint32_t*>(base + kOffTmp);
+    if (c.reach >= kListedReach) d.cell_head = d.tmp;
+    d = upload_view(d);
     d.counts = reinterpret_cast<uint32_t*>(base + kOffCounts);
     d.cell_start = reinterpret_cast<uint32_t*>(base + kOffCellStart);
     d.tile_sums = reinterpret_cast<uint32_t*>(base + kOffTileSums);

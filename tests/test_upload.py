@@ -1,5 +1,7 @@
 """Uploads and downloads at the sizes where their rows, warps and tile counting
 change: any particle order in, the same arrays out, and a consistent sort."""
+import time
+
 import numpy as np
 import pytest
 
@@ -58,3 +60,50 @@ def test_cells_of_any_size_sort_stably(cells, per_cell):
             s.step(1)  # the next histogram is the force pass's
             spos, svel, ids, keys = s.sortedState()
             assert (np.diff(keys.astype(np.int64)) >= 0).all() and s.checkState()["cell_table_mismatch"] == 0
+
+
+@pytest.mark.parametrize("cells", [1, 2, 3])
+@pytest.mark.parametrize("n", [2047, 2048, 5000])
+def test_crowds_in_the_border_cells(oracle, n, cells):
+    """A third of the positions outside the box, in few border cells: the sorted order and the first sub-steps, at the
+    sizes where the sort's form changes."""
+    rng = np.random.default_rng(n)
+    pos = rng.random((n, 3)).astype(np.float32)
+    far = rng.permutation(n)[:n // 3]
+    pos[far] = (np.array([7.0, -3.0, 7.0]) + rng.random((n // 3, 3))).astype(np.float32)
+    prm = params_16k(cellsPerH=cells)
+    st = oracle.State(pos)
+    keys, _ = st.sort(prm.to_c())
+    with SPHSolver(prm) as s:
+        s.setParticles(pos)
+        _, _, ids, k = s.sortedState()
+        np.testing.assert_array_equal(ids, st.ids)
+        np.testing.assert_array_equal(k, keys)
+        s.setParams(params_16k(cellsPerH=cells, boxMax=(0.5, 0.5, 0.5)))  # more of them outside
+        s.setParams(prm)
+        s.setParticles(pos)
+        s.step(2)
+        got = s.getState()
+    st = oracle.State(pos)
+    st.step(prm.to_c(), 2)
+    for a, b in zip(got, st.original_order()):
+        assert np.array_equal(a.view(np.uint32), b.view(np.uint32))
+
+
+def test_an_upload_into_one_cell_takes_no_serial_walk():
+    """32,768 particles beside the box in one border cell: within twice the time of the same with one cell per h, whose
+    sort never walks lists (0.8 ms both; walked as a list 2.7 ms)."""
+    n = 32768
+    pos = (5.0 + np.random.default_rng(1).random((n, 3))).astype(np.float32)
+    best = []
+    for cells in (1, 2):
+        with SPHSolver(params_16k(cellsPerH=cells)) as s:
+            t = []
+            for _ in range(10):
+                s.synchronize()
+                t0 = time.perf_counter()
+                s.setParticles(pos)
+                s.synchronize()
+                t.append(time.perf_counter() - t0)
+            best.append(min(t))
+    assert best[1] < 2.0 * best[0], best
