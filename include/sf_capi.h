@@ -186,7 +186,8 @@ typedef struct sf_device_view {
 SF_API sf_status sf_device_state(sf_ctx* ctx, sf_device_view* view);
 
 /* ---- stepping: makeReady() / advanceFrame() ----------------------------- */
-/* Build the uniform grid, sort the particles and capture the step graph. */
+/* Build the uniform grid, sort the particles and capture the graph of one
+ * sub-step. */
 SF_API sf_status sf_make_ready(sf_ctx* ctx);
 /* One sub-step; *dt_out receives the simulated time advanced.  With a fixed
  * time step the work is queued and the call does not wait; with the adaptive
@@ -196,10 +197,17 @@ SF_API sf_status sf_advance_frame(sf_ctx* ctx, float* dt_out);
  * summed in float, reach frame_time (the loop of Source/Simulator.cpp:46-51,
  * frame_time 0.0333333333) or max_substeps were taken.  Each frame is one CUDA
  * graph launch whose sub-step loop is a device-side conditional while node.
- * Waits; reports the simulated time and the sub-steps taken in total. */
+ * Waits; reports the simulated time and the sub-steps taken in total.  How a
+ * frame is run (threads per particle, sub-steps per loop) also goes by the
+ * contexts on the same GPU whose frames other threads run; the bits do not. */
 SF_API sf_status sf_advance_frames(sf_ctx* ctx, uint32_t frames, double frame_time, uint32_t max_substeps,
                                    double* sim_time_out, uint32_t* substeps_out);
-/* `nsteps` sub-steps, queued as replays of one captured step graph. */
+/* `nsteps` sub-steps, queued as replays of captured graphs of one or more
+ * sub-steps (a context's first call may queue the kernels themselves).  Scenes of
+ * fewer than 57,344 particles are stepped with several threads per particle
+ * unless other contexts of the process keep the same GPU busy: have queued
+ * sub-steps of as many particles in all, unfinished and not waited for.  The
+ * bits do not depend on it. */
 SF_API sf_status sf_step(sf_ctx* ctx, uint32_t nsteps);
 /* Wait for all queued work of the context. */
 SF_API sf_status sf_synchronize(sf_ctx* ctx);

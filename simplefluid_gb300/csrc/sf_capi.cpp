@@ -11,6 +11,8 @@
 #include <sys/mman.h>
 #include <unistd.h>
 
+#include <mutex>
+
 #include "sf_capi_impl.h"
 
 namespace sf {
@@ -206,6 +208,150 @@ void free_render(sf_ctx* ctx) {
     ctx->render_n = 0;
 }
 
+// Sub-steps that the contexts of this process have queued on a device.
+struct DeviceQueues {
+    std::mutex m;  // the list
+    sf::QueueMark* first = nullptr;
+    std::atomic<uint64_t> particles{0};  // of all marks
+};
+static DeviceQueues& queues_of(int device) {
+    static DeviceQueues per_device[64];
+    return per_device[device & 63];
+}
+
+static void set_mark(sf::QueueMark& mark, uint32_t n) {
+    const uint32_t old = mark.n.exchange(n, std::memory_order_relaxed);
+    if (old != n) queues_of(mark.device).particles.fetch_add((uint64_t)n - old, std::memory_order_relaxed);
+}
+
+void note_queued(sf_ctx* ctx) {
+    sf::QueueMark& mark = ctx->mark;
+    if (!mark.listed) {
+        mark.device = ctx->device;
+        mark.stream = ctx->stream;
+        DeviceQueues& q = queues_of(mark.device);
+        std::lock_guard<std::mutex> lock(q.m);
+        mark.next = q.first;
+        if (q.first) q.first->prev = &mark;
+        q.first = &mark;
+        mark.listed = true;
+    }
+    set_mark(mark, ctx->d.n);
+}
+
+CaptureGuard::CaptureGuard(sf_ctx* ctx) : ctx_(ctx) {
+    std::lock_guard<std::mutex> lock(queues_of(ctx->device).m);
+    ctx->mark.capturing = true;
+}
+CaptureGuard::~CaptureGuard() {
+    std::lock_guard<std::mutex> lock(queues_of(ctx_->device).m);
+    ctx_->mark.capturing = false;
+}
+
+static void unlist_mark(sf::QueueMark& mark) {
+    if (!mark.listed) return;
+    set_mark(mark, 0);
+    DeviceQueues& q = queues_of(mark.device);
+    std::lock_guard<std::mutex> lock(q.m);
+    (mark.prev ? mark.prev->next : q.first) = mark.next;
+    if (mark.next) mark.next->prev = mark.prev;
+    mark.prev = mark.next = nullptr;
+    mark.listed = false;
+}
+
+// Particles of the sub-steps that the other contexts of the process have queued
+// on the GPU.  As the marks have it, which costs nothing but counts work that has
+// ended without its context being waited for (a program may wait by other means):
+static uint64_t marked_others(sf_ctx* ctx) {
+    return queues_of(ctx->device).particles.load(std::memory_order_relaxed) -
+           ctx->mark.n.load(std::memory_order_relaxed);
+}
+
+// as the streams have it, up to the number that matters (about a microsecond;
+// idle streams' marks are cleared).
+static uint64_t busy_others(sf_ctx* ctx) {
+    uint64_t busy = 0;
+    // another thread may be capturing: looking at a stream is no part of that
+    cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+    cudaThreadExchangeStreamCaptureMode(&mode);
+    {
+        DeviceQueues& q = queues_of(ctx->device);
+        std::lock_guard<std::mutex> lock(q.m);
+        for (sf::QueueMark* o = q.first; o && busy < sf::kDensityTeamScene; o = o->next) {
+            const uint32_t n = o->n.load(std::memory_order_relaxed);
+            if (o == &ctx->mark || !n || o->capturing) continue;
+            // a stream that a program captures must not be queried
+            cudaStreamCaptureStatus captured = cudaStreamCaptureStatusActive;
+            if (cudaStreamIsCapturing(o->stream, &captured) != cudaSuccess || captured != cudaStreamCaptureStatusNone)
+                continue;
+            if (cudaStreamQuery(o->stream) == cudaErrorNotReady)
+                busy += n;
+            else
+                set_mark(*o, 0);
+        }
+    }
+    cudaThreadExchangeStreamCaptureMode(&mode);
+    if (cudaPeekAtLastError() == cudaErrorNotReady) cudaGetLastError();  // the answer, not an error
+    return busy;
+}
+
+// The kernels of the sub-steps about to be queued.  The teams of the small
+// scenes shorten one scene's time but take up to twice the GPU's: contexts that
+// step 19,000 particles each, none waited for, make, with teams / without, 2.9e9 /
+// 3.0e9 particle-updates/s two at a time, 3.2e9 / 3.9e9 four, 3.0e9 / 4.6e9
+// thirty-two, 2.7e9 / 4.8e9 all 256.  Contexts that are waited for in turn have
+// the GPU to themselves and keep their teams.  The results are the same bits.
+// The streams are looked at once for kTrustShared calls.
+constexpr uint32_t kTrustShared = 16;
+static bool teams_alone(sf_ctx* ctx) {  // teams where no other context is busy
+    ctx->d.shared = false;
+    return sf::team_scene(ctx->d, ctx->c, sf::kDensityTeamScene);
+}
+static void choose_shared(sf_ctx* ctx) {
+    constexpr uint64_t kFills = sf::kDensityTeamScene;
+    if (!teams_alone(ctx) || marked_others(ctx) < kFills) {
+        ctx->trust_shared = 0;
+        return;
+    }
+    if (!ctx->trust_shared && busy_others(ctx) >= kFills) ctx->trust_shared = kTrustShared;
+    if (!ctx->trust_shared) return;
+    --ctx->trust_shared;
+    ctx->d.shared = true;
+}
+
+// The same for frames, and whether they run their sub-steps in runs.  Calls of
+// sf_advance_frames wait for their frames, so those of one thread never share the
+// GPU; what counts is the contexts that other threads ran frames of last.  That
+// they do so at this moment would be a better measure, but one that changes from
+// call to call: a frame's graph takes far longer to make beside others' frames
+// than the frame itself.  More than 16 frames do not run at a time.  Where those
+// that do fill the GPU twice, one thread per particle is as fast or faster: ns per
+// particle update with teams / without, 8,000 particles from 8, 12 and 16 threads
+// 0.54 / 0.75, 0.50 / 0.58, 0.48 / 0.48; 12,000 0.46 / 0.53, 0.46 / 0.45, 0.45 /
+// 0.41; 25,000 from 4, 8 and 16 0.45 / 0.46, 0.46 / 0.39, 0.44 / 0.32.
+constexpr uint32_t kFramesAtATime = 16, kFramesFillGpu = 2 * sf::kDensityTeamScene;
+static bool choose_frame_kernels(sf_ctx* ctx) {
+    static std::atomic<uint32_t> threads{0};
+    thread_local const uint32_t thread = threads.fetch_add(1, std::memory_order_relaxed) + 1;
+    note_queued(ctx);
+    uint64_t particles = 0;
+    uint32_t contexts = 0;
+    {
+        DeviceQueues& q = queues_of(ctx->device);
+        std::lock_guard<std::mutex> lock(q.m);
+        ctx->mark.frame_thread = thread;
+        ctx->mark.frame_n = ctx->d.n;
+        for (const sf::QueueMark* o = q.first; o; o = o->next) {
+            if (!o->frame_thread || o->frame_thread == thread) continue;
+            particles += o->frame_n;
+            ++contexts;
+        }
+    }
+    if (contexts >= kFramesAtATime) particles = particles / contexts * (kFramesAtATime - 1);
+    ctx->d.shared = teams_alone(ctx) && ctx->d.n + particles >= kFramesFillGpu;
+    return contexts < sf::kFrameContexts;
+}
+
 static void destroy_retired(sf_ctx* ctx) {
     for (uint32_t k = 0; k < ctx->nretired; ++k) cudaGraphExecDestroy(ctx->retired[k]);
     ctx->nretired = 0;
@@ -225,15 +371,18 @@ void retire_graph(sf_ctx* ctx, cudaGraphExec_t& g) {
 
 sf_status wait_stream(sf_ctx* ctx) {
     SF_CUDA(cudaStreamSynchronize(ctx->stream));
+    set_mark(ctx->mark, 0);
     destroy_retired(ctx);
     return SF_OK;
 }
 
 void drop_graph(sf_ctx* ctx) {
-    retire_graph(ctx, ctx->step_graph);
-    retire_graph(ctx, ctx->run_graph);
-    retire_graph(ctx, ctx->call_graph);
-    ctx->call_steps = ctx->last_steps = ctx->repeats = 0;
+    for (sf::StepGraphs& g : ctx->graphs) {
+        retire_graph(ctx, g.step);
+        retire_graph(ctx, g.run);
+        retire_graph(ctx, g.call);
+        g = sf::StepGraphs{};
+    }
     ctx->stepped = false;
     ++ctx->gen;
 }
@@ -378,6 +527,7 @@ sf_status capture_steps(sf_ctx* ctx, uint32_t nsteps, cudaGraphExec_t* out) {
     // the gather records' persisting-L2 window (reserved outside the capture)
     if (ctx->d.tune.l2_window) sf::reserve_persisting_l2((size_t)ctx->d.n * 2 * sizeof(float4));
     cudaGraph_t g = nullptr;
+    CaptureGuard guard(ctx);
     SF_CUDA(cudaStreamBeginCapture(ctx->stream, cudaStreamCaptureModeThreadLocal));
     for (uint32_t s = 0; s < nsteps; ++s) enqueue_full_step(ctx);
     cudaError_t e = cudaStreamEndCapture(ctx->stream, &g);
@@ -409,63 +559,38 @@ constexpr uint32_t kFirstSteps = 32;
 constexpr uint32_t kCallSteps = 32, kLongCall = 256;
 
 // The graph of a whole call, or of kCallSteps of its sub-steps, where it pays.
-static sf_status need_call_graph(sf_ctx* ctx, uint32_t nsteps) {
-    ctx->repeats = nsteps == ctx->last_steps ? ctx->repeats + 1 : 0;
-    ctx->last_steps = nsteps;
+static sf_status need_call_graph(sf_ctx* ctx, sf::StepGraphs& g, uint32_t nsteps) {
+    g.repeats = nsteps == g.last_steps ? g.repeats + 1 : 0;
+    g.last_steps = nsteps;
     const uint32_t len = std::min(nsteps, kCallSteps);
-    if (len <= kRunSteps || len == ctx->call_steps || (ctx->repeats < 2 && nsteps < kLongCall)) return SF_OK;
-    retire_graph(ctx, ctx->call_graph);
-    ctx->call_steps = 0;
-    SF_TRY(capture_steps(ctx, len, &ctx->call_graph));
-    ctx->call_steps = len;
+    if (len <= kRunSteps || len == g.call_steps || (g.repeats < 2 && nsteps < kLongCall)) return SF_OK;
+    retire_graph(ctx, g.call);
+    g.call_steps = 0;
+    SF_TRY(capture_steps(ctx, len, &g.call));
+    g.call_steps = len;
     return SF_OK;
-}
-
-// Whether other contexts' sub-steps share the GPU with this one's: between its
-// last calls and the calls before them, others stepped as many particles as
-// fill the GPU by themselves.  The teams of the small scenes shorten one scene's
-// time but take up to twice the GPU's: contexts that step 19,000 particles each
-// in turn make, with teams / without, 2.9e9 / 3.0e9 particle-updates/s two at a
-// time, 3.2e9 / 3.9e9 four, 3.0e9 / 4.6e9 thirty-two, 2.7e9 / 4.8e9 all 256.
-// Four calls in a row decide, so that contexts used by turns do not flip; the
-// results are the same bits.
-static void note_sharing(sf_ctx* ctx) {
-    static std::atomic<uint64_t> stepped_on[64];  // particles of all calls, per device
-    const uint64_t n = ctx->d.n;
-    const uint64_t before = stepped_on[ctx->device & 63].fetch_add(n, std::memory_order_relaxed);
-    const bool shared = ctx->stepped_at != 0 && before - ctx->stepped_at >= sf::kDensityTeamScene;
-    ctx->stepped_at = before + n;
-    if (n >= sf::kDensityTeamScene) return;
-    if (shared == ctx->d.shared) {
-        ctx->sharing_calls = 0;
-    } else if (++ctx->sharing_calls == 4) {
-        ctx->sharing_calls = 0;
-        drop_graph(ctx);
-        ctx->stepped = true;  // graphs again at once: kernels are queued directly behind uploads only
-        ctx->d.shared = shared;
-    }
 }
 
 sf_status launch_steps(sf_ctx* ctx, uint32_t nsteps) {
     uint32_t left = nsteps;
-    note_sharing(ctx);
-    SF_TRY(need_call_graph(ctx, nsteps));
-    const bool graphs =
-        ctx->stepped || ctx->step_graph || ctx->run_graph || nsteps > kFirstSteps || ctx->d.tune.l2_window;
+    choose_shared(ctx);
+    note_queued(ctx);
+    sf::StepGraphs& g = ctx->graphs[ctx->d.shared];
+    SF_TRY(need_call_graph(ctx, g, nsteps));
+    const bool graphs = ctx->stepped || g.step || g.run || nsteps > kFirstSteps || ctx->d.tune.l2_window;
     ctx->stepped = true;
-    if (ctx->call_graph)
-        for (; left >= ctx->call_steps; left -= ctx->call_steps) SF_CUDA(cudaGraphLaunch(ctx->call_graph, ctx->stream));
-    if (graphs && left >= kRunSteps) {
-        if (!ctx->run_graph) SF_TRY(capture_steps(ctx, kRunSteps, &ctx->run_graph));
-        for (; left >= kRunSteps; left -= kRunSteps) SF_CUDA(cudaGraphLaunch(ctx->run_graph, ctx->stream));
-    }
-    if (!left) return SF_OK;
     if (!graphs) {
         for (; left; --left) enqueue_full_step(ctx);
         return check_launch("step");
     }
-    if (!ctx->step_graph) SF_TRY(capture_steps(ctx, 1, &ctx->step_graph));
-    for (; left; --left) SF_CUDA(cudaGraphLaunch(ctx->step_graph, ctx->stream));
+    if (g.call)
+        for (; left >= g.call_steps; left -= g.call_steps) SF_CUDA(cudaGraphLaunch(g.call, ctx->stream));
+    if (left >= kRunSteps) {
+        if (!g.run) SF_TRY(capture_steps(ctx, kRunSteps, &g.run));
+        for (; left >= kRunSteps; left -= kRunSteps) SF_CUDA(cudaGraphLaunch(g.run, ctx->stream));
+    }
+    if (left && !g.step) SF_TRY(capture_steps(ctx, 1, &g.step));
+    for (; left; --left) SF_CUDA(cudaGraphLaunch(g.step, ctx->stream));
     return SF_OK;
 }
 
@@ -529,11 +654,12 @@ void release_ctx(sf_ctx* ctx) {
     if (ctx->aux) cudaStreamSynchronize(ctx->aux);
     free_trajectory(ctx);
     free_render(ctx);
-    retire_graph(ctx, ctx->frame_graph);
+    retire_graph(ctx, ctx->frames.exec);
     if (ctx->frame) cudaFree(ctx->frame);
     ctx->frame = nullptr;
     drop_graph(ctx);
     destroy_retired(ctx);
+    unlist_mark(ctx->mark);
     free_particles(ctx->d);
     free_grid(ctx->d);
     if (ctx->h_stage) cudaFreeHost(ctx->h_stage);
@@ -1019,7 +1145,8 @@ SF_API sf_status sf_make_ready(sf_ctx* ctx) {
     SF_RANGE("sf_make_ready");
     SF_TRY(need_sorted(ctx));
     SF_TRY(set_device(ctx));
-    if (!ctx->step_graph) SF_TRY(capture_steps(ctx, 1, &ctx->step_graph));
+    sf::StepGraphs& g = ctx->graphs[ctx->d.shared];
+    if (!g.step) SF_TRY(capture_steps(ctx, 1, &g.step));
     return SF_OK;
 }
 
@@ -1060,10 +1187,12 @@ static sf_status add_frame_loop(sf_ctx* ctx, cudaGraph_t g, std::vector<cudaGrap
 // One frame as a graph: reset the frame clock, then conditional while nodes:
 // runs of sub-steps (of the lengths a frame has room for), then single ones up
 // to the frame's end.
-static sf_status build_frame_graph(sf_ctx* ctx, double frame_time, uint32_t max_substeps, cudaGraphExec_t* out) {
+static sf_status build_frame_graph(sf_ctx* ctx, double frame_time, uint32_t max_substeps, bool with_runs,
+                                   cudaGraphExec_t* out) {
     // the gather records' persisting-L2 window (reserved outside the captures)
     if (ctx->d.tune.l2_window) sf::reserve_persisting_l2((size_t)ctx->d.n * 2 * sizeof(float4));
     cudaGraph_t g = nullptr;
+    CaptureGuard capturing(ctx);
     SF_CUDA(cudaGraphCreate(&g, 0));
     struct GraphGuard {
         cudaGraph_t g;
@@ -1075,7 +1204,7 @@ static sf_status build_frame_graph(sf_ctx* ctx, double frame_time, uint32_t max_
     sf::FrameLoop runs[2], single;
     uint32_t nruns = 0;
     for (const uint32_t run : sf::kFrameRuns) {
-        if (!(run * (double)ctx->c.dt < frame_time && run < max_substeps)) continue;
+        if (!with_runs || !(run * (double)ctx->c.dt < frame_time && run < max_substeps)) continue;
         runs[nruns].run = run;
         SF_CUDA(cudaGraphConditionalHandleCreate(&runs[nruns++].h, g, 0, cudaGraphCondAssignDefault));
     }
@@ -1102,17 +1231,21 @@ SF_API sf_status sf_advance_frames(sf_ctx* ctx, uint32_t frames, double frame_ti
     SF_TRY(need_sorted(ctx));
     SF_TRY(set_device(ctx));
     if (!(frame_time > 0.0) || max_substeps == 0) return fail(SF_ERR_INVALID_ARGUMENT, "need frame_time > 0, max_substeps > 0");
-    if (!ctx->frame_graph || ctx->frame_graph_gen != ctx->gen || ctx->frame_graph_time != frame_time ||
-        ctx->frame_graph_max != max_substeps) {
-        retire_graph(ctx, ctx->frame_graph);
-        SF_TRY(build_frame_graph(ctx, frame_time, max_substeps, &ctx->frame_graph));
-        ctx->frame_graph_gen = ctx->gen;
-        ctx->frame_graph_time = frame_time;
-        ctx->frame_graph_max = max_substeps;
+    const bool runs = choose_frame_kernels(ctx);
+    sf::FrameGraph& fg = ctx->frames;
+    if (!fg.exec || fg.gen != ctx->gen || fg.time != frame_time || fg.max != max_substeps ||
+        fg.shared != ctx->d.shared || fg.runs != runs) {
+        retire_graph(ctx, fg.exec);
+        SF_TRY(build_frame_graph(ctx, frame_time, max_substeps, runs, &fg.exec));
+        fg.gen = ctx->gen;
+        fg.time = frame_time;
+        fg.max = max_substeps;
+        fg.shared = ctx->d.shared;
+        fg.runs = runs;
     }
     SF_CUDA(cudaMemsetAsync(&ctx->frame->substeps, 0, sizeof(uint32_t), ctx->stream));
     SF_CUDA(cudaMemsetAsync(&ctx->frame->sim_time, 0, sizeof(double), ctx->stream));
-    for (uint32_t f = 0; f < frames; ++f) SF_CUDA(cudaGraphLaunch(ctx->frame_graph, ctx->stream));
+    for (uint32_t f = 0; f < frames; ++f) SF_CUDA(cudaGraphLaunch(fg.exec, ctx->stream));
     sf::FrameState fs;
     SF_CUDA(cudaMemcpyAsync(&fs, ctx->frame, sizeof(fs), cudaMemcpyDeviceToHost, ctx->stream));
     SF_TRY(wait_stream(ctx));

@@ -106,6 +106,7 @@ sf_status build_segment_graph(sf_ctx* ctx, uint32_t len, cudaGraphExec_t* out) {
     const uint32_t n = d.n;
     cudaStream_t st = ctx->stream;
     cudaGraph_t g = nullptr;
+    CaptureGuard guard(ctx);
     SF_CUDA(cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal));
     sf::DeviceState r0 = d;
     r0.pos2 = t->stage;
@@ -282,6 +283,7 @@ SF_API sf_status sf_adjoint(sf_ctx* ctx, const float* dloss_dx, const float* dlo
     SF_TRY(upload_by_id(ctx, w.Vb, dloss_dv));
     SF_CUDA(cudaMemsetAsync(w.scalars, 0, 2 * sizeof(double), ctx->stream));
     const uint32_t nck = (uint32_t)t->ck.size();
+    note_queued(ctx);
     for (int64_t seg = (int64_t)nck - 1; seg >= 0; --seg) {
         const uint32_t s0 = (uint32_t)seg * t->ckpt, len = std::min(t->nsteps, s0 + t->ckpt) - s0;
         cudaGraphExec_t g = nullptr;

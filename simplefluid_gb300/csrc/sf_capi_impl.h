@@ -50,6 +50,33 @@ struct Trajectory {
     float* target = nullptr;
     double* hpartial = nullptr;
 };
+
+// Graphs of a context's sub-steps.
+struct StepGraphs {
+    cudaGraphExec_t step = nullptr;  // one sub-step
+    cudaGraphExec_t run = nullptr;   // kRunSteps sub-steps
+    cudaGraphExec_t call = nullptr;  // call_steps sub-steps
+    uint32_t call_steps = 0, last_steps = 0, repeats = 0;  // the last call's sub-steps, and how often they repeated
+};
+// A device frame's graph and what it was made for.
+struct FrameGraph {
+    cudaGraphExec_t exec = nullptr;
+    uint64_t gen = 0;
+    double time = 0.0;
+    uint32_t max = 0;
+    bool shared = false, runs = false;
+};
+// The particles of the sub-steps that a context has queued and not waited for
+// (see busy_others in sf_capi.cpp); linked into a list per device.
+struct QueueMark {
+    std::atomic<uint32_t> n{0};
+    cudaStream_t stream = nullptr;
+    int device = 0;
+    QueueMark *prev = nullptr, *next = nullptr;
+    // under the list's lock
+    bool listed = false, capturing = false;
+    uint32_t frame_thread = 0, frame_n = 0;  // the thread that ran frames of the context last (from 1), and their particles
+};
 }  // namespace sf
 
 struct sf_ctx {
@@ -66,26 +93,20 @@ struct sf_ctx {
     // tables (Grace: NVLink-C2C with address translation): -1 unknown, 0, 1
     int host_direct = -1;
     uint32_t* d_report = nullptr;  // sf_check_state counters
-    cudaGraphExec_t step_graph = nullptr;  // one sub-step
-    cudaGraphExec_t run_graph = nullptr;   // kRunSteps sub-steps
-    cudaGraphExec_t call_graph = nullptr;  // call_steps sub-steps
+    sf::StepGraphs graphs[2];      // by d.shared: for a GPU of its own, and a shared one
+    sf::QueueMark mark;
+    uint32_t trust_shared = 0;     // calls for which the last look at the other contexts holds
     // graphs given up while queued work may still use them: destroyed after a
     // wait for the stream
     cudaGraphExec_t retired[8] = {};
     uint32_t nretired = 0;
-    uint32_t call_steps = 0, last_steps = 0, repeats = 0;  // the last call's sub-steps, and how often they repeated
-    uint64_t stepped_at = 0;               // see note_sharing
-    uint32_t sharing_calls = 0;
-    bool stepped = false;                  // a call stepped since the graphs were last dropped
+    bool stepped = false;  // a call stepped since the graphs were last dropped
     bool sorted = false;  // particles uploaded and cell-sorted
     float* h_stage = nullptr;  // pinned staging for pageable caller buffers
     size_t h_stage_bytes = 0;
     sf::Trajectory* traj = nullptr;  // differentiable runs (sf_forward / sf_adjoint)
     sf::FrameState* frame = nullptr;  // device sub-step / frame state
-    cudaGraphExec_t frame_graph = nullptr;
-    uint64_t frame_graph_gen = 0;
-    double frame_graph_time = 0.0;
-    uint32_t frame_graph_max = 0;
+    sf::FrameGraph frames;
     // render buffers (sf_render)
     int render_w = 0, render_h = 0;
     uint32_t render_n = 0;
@@ -171,6 +192,19 @@ void drop_graph(sf_ctx* ctx);
 void retire_graph(sf_ctx* ctx, cudaGraphExec_t& g);
 // Waits for the context's stream.
 sf_status wait_stream(sf_ctx* ctx);
+// Counts the context's sub-steps as queued on the GPU until its stream is waited for.
+void note_queued(sf_ctx* ctx);
+// While it lives the context's stream may be captured: no other thread looks at it.
+class CaptureGuard {
+public:
+    explicit CaptureGuard(sf_ctx* ctx);
+    ~CaptureGuard();
+    CaptureGuard(const CaptureGuard&) = delete;
+    CaptureGuard& operator=(const CaptureGuard&) = delete;
+
+private:
+    sf_ctx* ctx_;
+};
 // Kernel choices by particle count, unless the caller set them explicitly.
 void apply_size_defaults(sf_ctx* ctx);
 

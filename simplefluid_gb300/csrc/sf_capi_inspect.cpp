@@ -176,10 +176,11 @@ SF_API sf_status sf_step_timed(sf_ctx* ctx, uint32_t nsteps, uint64_t flush_byte
     if (flush_bytes) SF_CUDA(dev_malloc(&flush.p, flush_bytes));
     EventSet ev;
     SF_CUDA(ev.create(2 * (size_t)nsteps));
+    note_queued(ctx);
     for (uint32_t i = 0; i < nsteps; ++i) {
         if (flush_bytes) SF_CUDA(cudaMemsetAsync(flush.p, (int)(i & 0xff), flush_bytes, ctx->stream));
         SF_CUDA(cudaEventRecord(ev.ev[2 * i], ctx->stream));
-        SF_CUDA(cudaGraphLaunch(ctx->step_graph, ctx->stream));
+        SF_CUDA(cudaGraphLaunch(ctx->graphs[ctx->d.shared].step, ctx->stream));
         SF_CUDA(cudaEventRecord(ev.ev[2 * i + 1], ctx->stream));
     }
     SF_TRY(wait_stream(ctx));

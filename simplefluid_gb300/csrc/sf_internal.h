@@ -107,7 +107,7 @@ struct DeviceState {
     uint8_t* nbr_wide = nullptr;   // SF_LIST_TILE16: per warp tile (kNbWarpTile particles), 1 where it holds 32-bit entries
     float4* pv = nullptr;          // 2 per particle (32 bytes): (x, vx, y, vy), (z, vz, p, 1/rho)
     float4* sums = nullptr;        // optional: per particle (AP, 0), (AV, 0) of the force pass (adjoint recording)
-    bool shared = false;           // other contexts step on the GPU in between: no team passes
+    bool shared = false;           // other contexts keep the GPU busy: no team passes
     FrameState* frame = nullptr;   // adaptive sub-steps read dt here and raise the maxima
     // grid
     uint32_t ncells = 0, ncells_pad = 0;
@@ -293,6 +293,12 @@ struct FrameLoop {
 // single sub-steps, 5280 in runs of 4, 5050 of 8, 4970 of 16.  Long steps fill a
 // frame with few (none of 16, some of 4), so there are two lengths.
 constexpr uint32_t kFrameRuns[2] = {16, 4};
+// Where other threads run frames of this many contexts or more, a frame has the
+// loop of single sub-steps alone: more than eight graphs of several while nodes at a time
+// get in each other's way.  Frames of 1,331 particles from 8, 10 and 16 threads, ns
+// per particle update, runs / single: 2.1 / 2.5, 3.1 / 2.1, 3.2 / 1.4; of 4,000
+// 0.83 / 1.07, 1.16 / 0.98, 1.37 / 0.79.
+constexpr uint32_t kFrameContexts = 8;
 // resets the frame clock; decides whether the loops of runs are entered
 void launch_frame_begin(FrameState* fs, const FrameLimits& l, const FrameLoop& first, const FrameLoop& second,
                         cudaStream_t s);

@@ -1,6 +1,8 @@
 """Many contexts with long queues of sub-steps that change their graphs while
 they are queued: every context's state is that of a run by itself."""
 
+import threading
+
 import numpy as np
 import pytest
 
@@ -66,3 +68,38 @@ def test_hundreds_of_contexts_in_bursts_and_in_turn():
             for _ in range(steps):
                 one.advanceFrame()
             same_bits(got[k], one.getState())
+
+
+def test_device_frames_on_many_threads():
+    """Frames of 12 contexts at once (more than run their sub-steps in runs) equal those of one after the other."""
+    prm = params_16k(timeStep=2e-4)
+    state = [cloud(900 + 61 * k, k) for k in range(12)]
+
+    def frames(s):
+        return [s.advanceFrames(2, f * 2e-4, 1000) for f in (7.5, 21.0, 21.0, 40.0)]
+
+    want = []
+    for x in state:
+        with SPHSolver(prm) as s:
+            s.setParticles(x)
+            want.append((frames(s), s.getState()))
+    ctxs = [SPHSolver(prm) for _ in state]
+    try:
+        for s, x in zip(ctxs, state):
+            s.setParticles(x)
+        times = [None] * 12
+
+        def run(k):
+            times[k] = frames(ctxs[k])
+
+        threads = [threading.Thread(target=run, args=(k,)) for k in range(12)]
+        for t in threads:
+            t.start()
+        for t in threads:
+            t.join()
+        for s, t, (want_times, want_state) in zip(ctxs, times, want):
+            assert t == want_times
+            same_bits(s.getState(), want_state)
+    finally:
+        for s in ctxs:
+            s.close()

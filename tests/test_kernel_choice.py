@@ -2,6 +2,7 @@
 import os
 import subprocess
 import sys
+import threading
 
 import pytest
 
@@ -101,3 +102,64 @@ def test_no_teams_where_the_lists_overflow_at_rest(ratio, team, cells):
     with SPHSolver(params_16k(kernelRadius=0.01 * ratio, cellsPerH=cells)) as s:
         s.setParticles(cloud(2000, 1))
         assert kernels(s)[:2] == (("density_team", "force_team") if team else ("density_256", "force_128_gather4"))
+
+
+@pytest.fixture
+def four():
+    """Four scenes of 30,000 particles: any two of them fill the GPU."""
+    prm = params_16k(particleRadius=0.005, kernelRadius=0.02)
+    solvers = [SPHSolver(prm) for _ in range(4)]
+    for k, s in enumerate(solvers):
+        s.setParticles(cloud(30000, k))
+        s.step(1)
+        s.synchronize()
+    yield solvers
+    for s in solvers:
+        s.close()
+
+
+def teams(s):
+    return kernels(s)[0] == "density_team"
+
+
+def test_contexts_that_keep_the_gpu_busy_take_one_thread_per_particle(four):
+    for _ in range(20):
+        for s in four:
+            s.step(20)
+    assert not any(teams(s) for s in four)
+    for s in four:
+        s.synchronize()
+    four[0].step(1)
+    assert teams(four[0])
+
+
+@pytest.mark.parametrize("wait", ["synchronize", "device"])
+def test_contexts_waited_for_in_turn_keep_their_teams(four, wait):
+    torch = pytest.importorskip("torch")
+    big = SPHSolver(params_16k(particleRadius=0.0025, kernelRadius=0.01))
+    big.setParticles(cloud(300000, 9, 0.4))
+    try:
+        for _ in range(8):
+            for s in (big, *four):
+                s.step(2)
+                s.synchronize() if wait == "synchronize" else torch.cuda.synchronize()
+                assert s is big or teams(s)
+    finally:
+        big.close()
+
+
+def test_frames_of_several_threads_take_one_thread_per_particle(four):
+    for _ in range(2):  # one after the other on this thread
+        for s in four:
+            s.advanceFrames(1, 3e-4, 100)
+            assert teams(s)
+    for _ in range(2):
+        threads = [threading.Thread(target=s.advanceFrames, args=(1, 3e-4, 100)) for s in four]
+        for t in threads:
+            t.start()
+        for t in threads:
+            t.join()
+    assert not any(teams(s) for s in four)
+    for s in four:  # this thread's again
+        s.advanceFrames(1, 3e-4, 100)
+    assert teams(four[3])
