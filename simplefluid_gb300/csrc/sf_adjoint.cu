@@ -169,7 +169,8 @@ __device__ __forceinline__ void adj_pair(float h, const AdjRec& k, const AdjRec&
 
 // The same of two neighbours a and b at once (`va`, `vb` clear: none, its
 // terms are zeros), a's added before b's, without the compiler's root and
-// divisions (see root_quotient): the packed halves are the position and the
+// divisions (see root_recip; the range is kFastR2Min to kAdjHMax^2, the numerators
+// are zero or at least kAdjTiny): the packed halves are the position and the
 // velocity side of one neighbour in the differences, dot products and sums,
 // and the two neighbours in between.  Signs differ from adj_pair's where that
 // saves an operation; every rounding is the same.
@@ -181,24 +182,17 @@ struct AdjPairSums {
     float nearest = 1.f;     // smallest r^2 so far
     uint32_t tiny = ~0u;     // smallest 2 bits(|numerator|) - 1 so far (numerators that are zero pass)
 };
-__device__ __forceinline__ F2 quotient2(F2 num, F2 minus_den, F2 recip) {
-    const F2 q0 = mul2(num, recip);
-    return fma2(fma2(minus_den, q0, num), recip, q0);
-}
 __device__ __forceinline__ void adj_pair2(float h, const F2 k[3], float pk, F2 invk, const PairRec& ck, const AdjRec& a,
                                           const AdjRec& b, bool va, bool vb, AdjPairSums& o) {
-    const F2 flip = f2(-1.f, 1.f), bias = f2(2.8421709e-14f, 2.8421709e-14f), one = f2(1.f, 1.f);
+    const F2 flip = f2(-1.f, 1.f);
     // (xk - xj, vj - vk); k holds (xk, -vk)
     const F2 ax = fma2(a.s.x, flip, k[0]), ay = fma2(a.s.y, flip, k[1]), az = fma2(a.s.z, flip, k[2]);
     const F2 bx = fma2(b.s.x, flip, k[0]), by = fma2(b.s.y, flip, k[1]), bz = fma2(b.s.z, flip, k[2]);
     const float ra = va ? square3(ax, ay, az) : 1.f, rb = vb ? square3(bx, by, bz) : 1.f;
     o.nearest = fminf(o.nearest, fminf(ra, rb));
     const F2 n2 = f2(-ra, -rb), y0 = f2(rsqrt_approx(ra), rsqrt_approx(rb));
-    const F2 ns = mul2(n2, y0);
-    const F2 nr = fma2(fma2(ns, ns, n2), mul2(y0, f2(0.5f, 0.5f)), ns);  // -r
-    const F2 y = fma2(add2(fma2(nr, y0, one), bias), y0, y0);            // 1 / r
-    const F2 z0 = mul2(y0, y0);
-    const F2 y2 = fma2(add2(fma2(n2, z0, one), bias), z0, z0);           // 1 / r^2
+    const RootRecip root = root_recip(n2, y0);
+    const F2 nr = root.nr, y = root.y, y2 = recip_step(n2, mul2(y0, y0));  // -r, 1 / r, 1 / r^2
     const float2 hr1 = unpack(add2(f2(h, h), nr));
     const F2 hr = f2(va ? hr1.x : 0.f, vb ? hr1.y : 0.f);  // zero weights where there is no neighbour
     const F2 q = quotient2(hr, nr, y);

@@ -563,38 +563,54 @@ __device__ __forceinline__ void ld_rec(const float4* __restrict__ p, PairRec& r)
                      : "l"(p));
 }
 
-// The distance and its quotient of two pairs, from their r^2.  They are not
-// the compiler's root and division: those branch on their operand's range,
-// which keeps two neighbours' chains from interleaving, and start from two
-// separate approximations.  Here both come from one approximation of
-// 1/sqrt(r^2): a Newton step in residual form for the root, one for its
-// reciprocal, then Markstein's quotient correction (P. Markstein, "Computation
-// of elementary functions on the IBM RISC System/6000 processor", 1990), all
-// on both pairs at once.  Over the stated range the results are the IEEE ones:
-// checked for every float r^2 (root), and for every quotient close enough to a
-// rounding boundary to be in doubt (118,635,758 numerators over all roots; the
-// error before the last rounding is under 1.5 * 2^-24 of a unit, so a quotient
-// further than that from a boundary cannot round wrong).
-// A coincident neighbour (r^2 = 0, the particle itself included) takes
-// r = 2^-45, so that h - r == h.
+// Roots, reciprocals and quotients of two pairs at once.  They are not the
+// compiler's root and division: those branch on their operand's range, which
+// keeps two neighbours' chains from interleaving, and start from separate
+// approximations.  Here all come from one approximation of 1/sqrt(r^2): a Newton
+// step in residual form for the root, one for its reciprocal and one for the
+// square's, then Markstein's quotient correction (P. Markstein, "Computation of
+// elementary functions on the IBM RISC System/6000 processor", 1990).
+//
+// Roots and quotients are the IEEE ones over the stated range
+// (tests/test_rounding.py).  The root is compared for every float there, and both
+// reciprocals are within (1/2 + 2^-20) of their last place of the exact value.  A
+// quotient is then off by less than 2^-22 (1 + 2^-18) of its last place before its
+// last rounding, so it can only round wrong where it lies that close to the
+// middle between two floats; these numerators are enumerated for every denominator.
+__device__ __forceinline__ F2 recip_step(F2 minus_den, F2 y) {
+    // the 2^-45 settles the reciprocal of a denominator one place below a power of
+    // two, which would round down
+    const F2 e = add2(fma2(minus_den, y, f2(1.f, 1.f)), f2(2.8421709e-14f, 2.8421709e-14f));
+    return fma2(e, y, y);
+}
+struct RootRecip {
+    F2 nr, y;  // -r, 1 / r
+};
+__device__ __forceinline__ RootRecip root_recip(F2 minus_r2, F2 y0) {  // y0: about 1 / r
+    const F2 ns = mul2(minus_r2, y0);                                     // -r^2 y0
+    const F2 d = fma2(ns, ns, minus_r2);                                  // residual (r^2 y0)^2 - r^2
+    RootRecip o;
+    o.nr = fma2(d, mul2(y0, f2(0.5f, 0.5f)), ns);
+    o.y = recip_step(o.nr, y0);
+    return o;
+}
+__device__ __forceinline__ F2 quotient2(F2 num, F2 minus_den, F2 recip) {
+    const F2 q0 = mul2(num, recip);
+    return fma2(fma2(minus_den, q0, num), recip, q0);
+}
+// h - r and its quotient by r of two pairs, from their r^2.  A coincident
+// neighbour (r^2 = 0, the particle itself included) takes r = 2^-45, so that
+// h - r == h.
 struct RootQuotient {
     F2 hr;      // h - r
     float2 nq;  // -(h - r) / r
 };
 __device__ __forceinline__ RootQuotient root_quotient(F2 hh, float ra, float rb) {
     const float ca = fmaxf(ra, kFastR2Min), cb = fmaxf(rb, kFastR2Min);
-    const F2 n2 = f2(-ca, -cb), y0 = f2(rsqrt_approx(ca), rsqrt_approx(cb));
-    const F2 ns = mul2(n2, y0);                             // -r^2 y0
-    const F2 d = fma2(ns, ns, n2);                          // residual (r^2 y0)^2 - r^2
-    const F2 nr = fma2(d, mul2(y0, f2(0.5f, 0.5f)), ns);    // -r
-    // 1 / r; the 2^-45 settles the one reciprocal that this step would round
-    // down (r one place below a power of two)
-    const F2 e = add2(fma2(nr, y0, f2(1.f, 1.f)), f2(2.8421709e-14f, 2.8421709e-14f));
-    const F2 y = fma2(e, y0, y0);
+    const RootRecip r = root_recip(f2(-ca, -cb), f2(rsqrt_approx(ca), rsqrt_approx(cb)));
     RootQuotient o;
-    o.hr = add2(hh, nr);
-    const F2 q0 = mul2(o.hr, y);
-    const float2 q = unpack(fma2(fma2(nr, q0, o.hr), y, q0));
+    o.hr = add2(hh, r.nr);
+    const float2 q = unpack(quotient2(o.hr, r.nr, r.y));
     o.nq = make_float2(-q.x, -q.y);
     return o;
 }
