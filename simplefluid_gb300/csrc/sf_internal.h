@@ -182,9 +182,15 @@ void launch_rank_gather(const DeviceState& d, cudaStream_t s);
 // eight and are bucketed (k_scatter): lists were neither faster nor slower there
 // (20 sub-steps of 16,000 particles 681 against 683 us).
 constexpr int kListedReach = 2;
-// Larger grids keep the bucketing too: the launch counts for little there
-// (1,048,576 particles, 8 million cells: 224.3 us a sub-step with lists, 227.0
-// without) and the heads would be 32 MB more to keep.
+// Larger grids keep the bucketing too.  The heads take 4 bytes a cell (16 MB at the
+// limit, 32 MB for 1,048,576 particles) and save one launch, about 1.5 us, of steps
+// that are long there.  A sub-step in us, bucketing / lists (lattice; disordered):
+// 4.5 Mi cells, 300,000 particles 81.6 / 80.8; 110.4 / 110.7, 600,000 147.7 / 146.5;
+// 201.8 / 200.2; 7.6 Mi, 1,048,576 221.2 / 219.4; 321.9 / 319.4; 10.2 Mi, 3,345,599
+// 659.3 / 653.2; 959.8 / 951.6; three cells per h, 12.2 Mi, 236,987 100.0 / 99.0;
+// 123.4 / 123.5, 25.8 Mi, 1,048,576 268.6 / 267.2; 405.4 / 406.8.  Few particles in
+// a large grid would gain more (100,000 in 4.9 Mi, three per h: 55.2 / 52.4; 62.6 /
+// 57.7).
 constexpr uint32_t kListedCells = 4u << 20;
 // A list is walked entry by entry, so a crowded cell takes longer than bucketed
 // indices do: the sort of 200,000 particles in cells of 16 members 21 us against 25,
