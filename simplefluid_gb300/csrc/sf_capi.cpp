@@ -544,7 +544,9 @@ sf_status capture_steps(sf_ctx* ctx, uint32_t nsteps, cudaGraphExec_t* out) {
 // Sub-steps of one run graph.  Inside it the last kernel of a sub-step and the
 // first of the next are chained like any other two; between two graphs the
 // GPU drains.  20 sub-steps of 16,000 particles 393 -> 376 us, of 65,536
-// 852 -> 827, 10 of 236,987 973 -> 953, of 1,048,576 2314 -> 2285.
+// 852 -> 827, 10 of 236,987 973 -> 953, of 1,048,576 2314 -> 2285.  Calls that are
+// no multiple, single graphs / runs and single ones: 7 of 16,000 163 / 147, 19 401 /
+// 373; 7 of 65,536 281 / 274, 19 745 / 706.
 constexpr uint32_t kRunSteps = 5;
 // A first call of at most this many sub-steps queues the kernels themselves
 // (a later one's last few go through the graph of one sub-step):
